@@ -10,6 +10,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
@@ -17,7 +18,7 @@ namespace gbf {
 // accumulates it: sqrt(fma(z, z, fma(y, y, x*x))).
 __device__ __forceinline__ double face_smag(const double* __restrict__ a) {
   const double x = a[0], y = a[1], z = a[2];
-  return __dsqrt_rn(__fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
+  return sqrt_rn(__fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
 }
 
 // Face diffusivity: constant, per face, or linearly interpolated from cells
@@ -37,8 +38,7 @@ struct DiffSpec {
 __device__ __forceinline__ double cell_D(const DiffSpec& D, int c) {
   const double v = __ldg(D.cell + c);
   if (D.mode != 3) return v;
-  const double a = fabs(v);
-  return __ddiv_rn(1.0, a < 1e-30 ? 1e-30 : a);  // clamp(min) keeps NaN
+  return div_rn(1.0, clamp_abs_min(v));  // clamp(min) keeps NaN
 }
 
 __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q, bool internal) {
@@ -48,6 +48,50 @@ __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q,
   if (!internal) return dp;
   const double w = __ldg(D.w + f);
   return __dadd_rn(__dmul_rn(w, dp), __dmul_rn(__dsub_rn(1.0, w), cell_D(D, q)));
+}
+
+// (0 + sum over the cell's owner-side faces) + (sum over its neighbour-side
+// faces, from 0) of own(f) / nei(f), faces in slot (= ascending) order.  The
+// first term of a sum enters without an addition (first_term), and a sum that
+// started at +0.0 is never -0.0, so adding it to 0.0 is the identity.  Up to
+// four slots a side (hex and most polyhedral cells) have every face index and
+// every face value of the cell in flight at once.
+template <typename O, typename N>
+__device__ __forceinline__ double cell_face_sum(const gbf_layout& L, int c, O&& own, N&& nei) {
+  double so = 0.0, sn = 0.0;
+  if (L.n_faces == 0) return 0.0;
+  const CellSlots cs = cell_slots(L, c);
+  if (cs.wo <= 4 && cs.wn <= 4) {
+    int f[8];
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
+      f[4 + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = f[k] >= 0 ? own(f[k]) : 0.0;
+      v[4 + k] = f[4 + k] >= 0 ? nei(f[4 + k]) : 0.0;
+    }
+    if (f[0] >= 0) so = first_term(v[0]);
+    if (f[4] >= 0) sn = first_term(v[4]);
+#pragma unroll
+    for (int k = 1; k < 4; ++k) {
+      if (f[k] >= 0) so = __dadd_rn(so, v[k]);
+      if (f[4 + k] >= 0) sn = __dadd_rn(sn, v[4 + k]);
+    }
+  } else {
+    for (int k = 0; k < cs.wo; ++k) {
+      const int f = __ldg(L.slot_face + cs.base + 32 * k);
+      if (f >= 0) so = __dadd_rn(so, own(f));
+    }
+    for (int k = 0; k < cs.wn; ++k) {
+      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
+      if (f >= 0) sn = __dadd_rn(sn, nei(f));
+    }
+  }
+  return __dadd_rn(so, sn);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -60,8 +104,8 @@ __global__ void __launch_bounds__(kBlock)
   const int p = __ldg(own + f), q = __ldg(nei + f);
   double c = __dmul_rn(face_D(D, f, p, q, true), face_smag(areas + 3 * (size_t)f));
   c = __dmul_rn(c, __ldg(delta + f));
-  lower[f] = __ddiv_rn(-c, __ldg(V + p));
-  upper[f] = __ddiv_rn(-c, __ldg(V + q));
+  lower[f] = div_rn(-c, __ldg(V + p));
+  upper[f] = div_rn(-c, __ldg(V + q));
 }
 
 // diag[c] = ((0 + sum_own c/V) + sum_nei c/V) + sum_bnd c_b/V, using
@@ -74,20 +118,8 @@ __global__ void __launch_bounds__(kBlock)
                     int has_bnd, double* __restrict__ diag) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
-  double so = 0.0, sn = 0.0;
-  if (L.n_faces > 0) {
-    const CellSlots cs = cell_slots(L, c);
-    for (int k = 0; k < cs.wo; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * k);
-      if (f >= 0) so = __dadd_rn(so, -__ldg(lower + f));
-    }
-    for (int k = 0; k < cs.wn; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
-      if (f >= 0) sn = __dadd_rn(sn, -__ldg(upper + f));
-    }
-  }
-  double d = __dadd_rn(0.0, so);
-  d = __dadd_rn(d, sn);
+  double d = cell_face_sum(
+      L, c, [&](int f) { return -__ldg(lower + f); }, [&](int f) { return -__ldg(upper + f); });
   if (has_bnd) {
     double sb = 0.0;
     const double vc = __ldg(V + c);
@@ -95,7 +127,7 @@ __global__ void __launch_bounds__(kBlock)
       const int f = __ldg(bnd_face + k);
       double cb = __dmul_rn(face_D(D, f, c, c, false), face_smag(areas + 3 * (size_t)f));
       cb = __dmul_rn(cb, __ldg(delta + f));
-      sb = __dadd_rn(sb, __ddiv_rn(cb, vc));
+      sb = __dadd_rn(sb, div_rn(cb, vc));
     }
     d = __dadd_rn(d, sb);
   }
@@ -111,9 +143,9 @@ __global__ void __launch_bounds__(kBlock)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nint) return;
   const double F = __ldg(flux + f);
-  const bool pos = F >= 0.0;
-  lower[f] = __ddiv_rn(pos ? 0.0 : F, __ldg(V + __ldg(own + f)));
-  upper[f] = __ddiv_rn(pos ? F : 0.0, __ldg(V + __ldg(nei + f)));
+  const bool pos = not_negative(F);
+  lower[f] = div_rn(pos ? 0.0 : F, __ldg(V + __ldg(own + f)));
+  upper[f] = div_rn(pos ? F : 0.0, __ldg(V + __ldg(nei + f)));
 }
 
 // diag = (0 + sum_own (-F+)/V_P) + sum_nei |F-|/V_N
@@ -123,23 +155,16 @@ __global__ void __launch_bounds__(kBlock)
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
   const double vc = __ldg(V + c);
-  double so = 0.0, sn = 0.0;
-  if (L.n_faces > 0) {
-    const CellSlots cs = cell_slots(L, c);
-    for (int k = 0; k < cs.wo; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * k);
-      if (f < 0) continue;
-      const double F = __ldg(flux + f);
-      so = __dadd_rn(so, __ddiv_rn(-(F >= 0.0 ? F : 0.0), vc));
-    }
-    for (int k = 0; k < cs.wn; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
-      if (f < 0) continue;
-      const double F = __ldg(flux + f);
-      sn = __dadd_rn(sn, __ddiv_rn(fabs(F >= 0.0 ? 0.0 : F), vc));
-    }
-  }
-  diag[c] = __dadd_rn(__dadd_rn(0.0, so), sn);
+  diag[c] = cell_face_sum(
+      L, c,
+      [&](int f) {
+        const double F = __ldg(flux + f);
+        return div_rn(-(not_negative(F) ? F : 0.0), vc);
+      },
+      [&](int f) {
+        const double F = __ldg(flux + f);
+        return div_rn(fabs(not_negative(F) ? 0.0 : F), vc);
+      });
 }
 
 // Linear-interpolation weights w = |d_N| / (|d_P| + |d_N|) of internal faces
@@ -162,7 +187,7 @@ __global__ void __launch_bounds__(kBlock)
   }
   const double dP = face_smag(a), dN = face_smag(b);
   const double den = __dadd_rn(dP, dN);
-  w[f] = __ddiv_rn(dN, den > 1e-30 ? den : 1.0);
+  w[f] = div_rn(dN, above_tiny(den) ? den : 1.0);
 }
 
 }  // namespace gbf
@@ -269,10 +294,10 @@ __global__ void __launch_bounds__(kBlock)
   if (f >= nfaces) return;
   const int p = __ldg(own_all + f);
   const double sd = face_smag(areas + 3 * (size_t)f) * __ldg(delta + f);
-  double g = (__ldg(gd + p) - (f < nint ? __ldg(gl + f) : 0.0)) / __ldg(V + p);
+  double g = div_rn(__ldg(gd + p) - (f < nint ? __ldg(gl + f) : 0.0), __ldg(V + p));
   if (f < nint) {
     const int q = __ldg(nei + f);
-    g += (__ldg(gd + q) - __ldg(gu + f)) / __ldg(V + q);
+    g += div_rn(__ldg(gd + q) - __ldg(gu + f), __ldg(V + q));
   }
   gD[f] = sd * g;
 }
@@ -314,9 +339,10 @@ __global__ void __launch_bounds__(kBlock)
   double g;
   if (f < nint) {
     const int q = __ldg(nei + f);
-    g = (__ldg(x + q) - __ldg(x + p)) * (__ldg(lam + p) / __ldg(V + p) - __ldg(lam + q) / __ldg(V + q));
+    g = (__ldg(x + q) - __ldg(x + p)) *
+        (div_rn(__ldg(lam + p), __ldg(V + p)) - div_rn(__ldg(lam + q), __ldg(V + q)));
   } else {
-    g = -__ldg(lam + p) * __ldg(x + p) / __ldg(V + p);
+    g = div_rn(-__ldg(lam + p) * __ldg(x + p), __ldg(V + p));
   }
   g = scale * sd * g;
   gD[f] = accumulate ? gD[f] + g : g;
@@ -394,7 +420,12 @@ extern "C" int gbf_adjoint_face_grad_f64(const gbf_layout* L, int32_t n_faces_to
 // ---------------------------------------------------------------------------
 namespace gbf {
 
-__device__ __forceinline__ double clamp_volume(double v) { return v < 1e-30 ? 1e-30 : v; }
+__device__ __forceinline__ double clamp_volume(double v) {
+  // v < 1e-30 on the integer pipe: every negative value, and the positive ones below 1e-30
+  const long long b = __double_as_longlong(v), lo = __double_as_longlong(1e-30);
+  const bool nan = (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+  return (b < lo && !nan) ? 1e-30 : v;
+}
 
 __global__ void __launch_bounds__(kBlock)
     explicit_lap_kernel(gbf_layout L, const int32_t* __restrict__ bnd_ptr,
@@ -429,8 +460,7 @@ __global__ void __launch_bounds__(kBlock)
       sn = __dadd_rn(sn, -fl);
     }
   }
-  double y = __dadd_rn(0.0, so);
-  y = __dadd_rn(y, sn);
+  double y = __dadd_rn(so, sn);
   if (has_bnd) {
     double sb = 0.0;
     for (int k = __ldg(bnd_ptr + c); k < __ldg(bnd_ptr + c + 1); ++k) {
@@ -441,7 +471,7 @@ __global__ void __launch_bounds__(kBlock)
     }
     y = __dadd_rn(y, sb);
   }
-  out[c] = __ddiv_rn(y, clamp_volume(__ldg(V + c)));
+  out[c] = div_rn(y, clamp_volume(__ldg(V + c)));
 }
 
 // D-gradient per face (:570-600):
@@ -456,11 +486,11 @@ __global__ void __launch_bounds__(kBlock)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nfaces) return;
   const int p = __ldg(own_all + f);
-  const double gp = __ddiv_rn(__ldg(g + p), clamp_volume(__ldg(V + p)));
+  const double gp = div_rn(__ldg(g + p), clamp_volume(__ldg(V + p)));
   double a;
   if (f < nint) {
     const int q = __ldg(nei + f);
-    const double gq = __ddiv_rn(__ldg(g + q), clamp_volume(__ldg(V + q)));
+    const double gq = div_rn(__ldg(g + q), clamp_volume(__ldg(V + q)));
     a = __dmul_rn(__dsub_rn(gp, gq), __dsub_rn(__ldg(phi + q), __ldg(phi + p)));
   } else {
     a = __dmul_rn(gp, __ldg(phi + p));
@@ -477,20 +507,9 @@ __global__ void __launch_bounds__(kBlock)
                               double* __restrict__ gcell) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
-  double so = 0.0, sn = 0.0;
-  if (L.n_faces > 0) {
-    const CellSlots cs = cell_slots(L, c);
-    for (int k = 0; k < cs.wo; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * k);
-      if (f >= 0) so = __dadd_rn(so, __dmul_rn(__ldg(gface + f), 0.5));
-    }
-    for (int k = 0; k < cs.wn; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
-      if (f >= 0) sn = __dadd_rn(sn, __dmul_rn(__ldg(gface + f), 0.5));
-    }
-  }
-  double y = __dadd_rn(0.0, so);
-  y = __dadd_rn(y, sn);
+  double y = cell_face_sum(
+      L, c, [&](int f) { return __dmul_rn(__ldg(gface + f), 0.5); },
+      [&](int f) { return __dmul_rn(__ldg(gface + f), 0.5); });
   if (has_bnd) {
     double sb = 0.0;
     for (int k = __ldg(bnd_ptr + c); k < __ldg(bnd_ptr + c + 1); ++k)
@@ -592,27 +611,15 @@ __global__ void __launch_bounds__(kBlock)
                            const double* __restrict__ V, int has_bnd, double* __restrict__ src) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
-  double so = 0.0, sn = 0.0;
-  if (L.n_faces > 0) {
-    const CellSlots cs = cell_slots(L, c);
-    for (int k = 0; k < cs.wo; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * k);
-      if (f >= 0) so = __dadd_rn(so, -__ldg(phi + f));
-    }
-    for (int k = 0; k < cs.wn; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
-      if (f >= 0) sn = __dadd_rn(sn, __ldg(phi + f));
-    }
-  }
-  double y = __dadd_rn(0.0, so);
-  y = __dadd_rn(y, sn);
+  double y = cell_face_sum(
+      L, c, [&](int f) { return -__ldg(phi + f); }, [&](int f) { return __ldg(phi + f); });
   if (has_bnd) {
     double sb = 0.0;
     for (int k = __ldg(bnd_ptr + c); k < __ldg(bnd_ptr + c + 1); ++k)
       sb = __dadd_rn(sb, -__ldg(phi + __ldg(bnd_face + k)));
     y = __dadd_rn(y, sb);
   }
-  src[c] = __ddiv_rn(y, __ldg(V + c));
+  src[c] = div_rn(y, __ldg(V + c));
 }
 }  // namespace gbf
 

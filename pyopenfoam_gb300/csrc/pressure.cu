@@ -16,12 +16,12 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
 __device__ __forceinline__ double inv_abs_clamped(double a) {
-  const double m = fabs(a);
-  return __ddiv_rn(1.0, m > 1e-30 ? m : 1e-30);
+  return div_rn(1.0, max_abs_tiny(a));
 }
 
 // w*a + (1 - w)*b with each operation rounded.
@@ -31,7 +31,7 @@ __device__ __forceinline__ double lerp_w(double w, double a, double b) {
 
 __device__ __forceinline__ double fma_norm3(const double* __restrict__ a) {
   const double x = __ldg(a), y = __ldg(a + 1), z = __ldg(a + 2);
-  return __dsqrt_rn(__fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
+  return sqrt_rn(__fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -39,9 +39,8 @@ __global__ void __launch_bounds__(kBlock)
                 double* __restrict__ out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
-  const double m = fabs(__ldg(A + c));
-  const double d = m > 1e-30 ? m : 1e-30;
-  for (int k = 0; k < 3; ++k) out[3 * (size_t)c + k] = __ddiv_rn(__ldg(H + 3 * (size_t)c + k), d);
+  const double d = max_abs_tiny(__ldg(A + c));
+  for (int k = 0; k < 3; ++k) out[3 * (size_t)c + k] = div_rn(__ldg(H + 3 * (size_t)c + k), d);
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -80,19 +79,21 @@ __global__ void __launch_bounds__(kBlock)
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
   const int P = __ldg(own + f);
-  double s = 0.0;
+  double s;
   if (f < nint) {
     const int N = __ldg(nei + f);
     const double wf = w ? __ldg(w + f) : 0.5;
     for (int k = 0; k < 3; ++k) {
       const double hf = lerp_w(wf, __ldg(HbyA + 3 * (size_t)P + k), __ldg(HbyA + 3 * (size_t)N + k));
-      s = __dadd_rn(s, __dmul_rn(hf, __ldg(areas + 3 * (size_t)f + k)));
+      const double t = __dmul_rn(hf, __ldg(areas + 3 * (size_t)f + k));
+      s = k == 0 ? first_term(t) : __dadd_rn(s, t);
     }
     if (p) s = __dadd_rn(s, rc_term(f, own, nei, p, A, areas, delta, w));
   } else {
-    for (int k = 0; k < 3; ++k)
-      s = __dadd_rn(s, __dmul_rn(__ldg(HbyA + 3 * (size_t)P + k), __ldg(areas + 3 * (size_t)f + k)));
-    if (p) s = __dadd_rn(s, 0.0);
+    for (int k = 0; k < 3; ++k) {
+      const double t = __dmul_rn(__ldg(HbyA + 3 * (size_t)P + k), __ldg(areas + 3 * (size_t)f + k));
+      s = k == 0 ? first_term(t) : __dadd_rn(s, t);
+    }  // s + 0.0 of the Rhie-Chow form is s: a sum from +0.0 is never -0.0
   }
   phi[f] = s;
 }
@@ -125,39 +126,59 @@ __global__ void __launch_bounds__(kBlock)
                             double alpha, double* __restrict__ U) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
+  // The cell itself is the owner (neighbour) of its owner-side (neighbour-
+  // side) faces and slot_col names the cell across, so a face costs one index
+  // pair and one p gather, not the four loads of its owner / neighbour entry.
+  const double pc = __ldg(p + c);
   double g[3] = {0.0, 0.0, 0.0};
   if (L.n_faces > 0) {
     const CellSlots cs = cell_slots(L, c);
+    bool first = true;
     for (int side = 0; side < 2; ++side) {
       const int k0 = side == 0 ? 0 : cs.wo, k1 = side == 0 ? cs.wo : cs.wo + cs.wn;
-      for (int k = k0; k < k1; ++k) {
-        const int f = __ldg(L.slot_face + cs.base + 32 * k);
-        if (f < 0) continue;
-        const int P = __ldg(L.owner + f), N = __ldg(L.neighbour + f);
-        const double pf = lerp_w(__ldg(w + f), __ldg(p + P), __ldg(p + N));
-        for (int q = 0; q < 3; ++q) {
-          const double t = __dmul_rn(pf, __ldg(areas + 3 * (size_t)f + q));
-          g[q] = __dadd_rn(g[q], side == 0 ? t : -t);
+      for (int kb = k0; kb < k1; kb += 4) {
+        int f[4];
+        double wf[4], pn[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int i = cs.base + 32 * (kb + j);
+          f[j] = kb + j < k1 ? __ldg(L.slot_face + i) : -1;
+          const int q = kb + j < k1 ? __ldg(L.slot_col + i) : -1;
+          pn[j] = q >= 0 ? __ldg(p + q) : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wf[j] = f[j] >= 0 ? __ldg(w + f[j]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (f[j] < 0) continue;
+          const double pf = side == 0 ? lerp_w(wf[j], pc, pn[j]) : lerp_w(wf[j], pn[j], pc);
+          const double pfs = side == 0 ? pf : -pf;  // a sign commutes with the rounding
+          for (int q = 0; q < 3; ++q) {
+            const double t = __dmul_rn(pfs, __ldg(areas + 3 * (size_t)f[j] + q));
+            g[q] = first ? first_term(t) : __dadd_rn(g[q], t);
+          }
+          first = false;
         }
       }
     }
   }
-  const double pc = __ldg(p + c);
   for (int i = __ldg(bnd_ptr + c), e = __ldg(bnd_ptr + c + 1); i < e; ++i) {
     const int f = __ldg(bnd_face + i);
     for (int q = 0; q < 3; ++q) g[q] = __dadd_rn(g[q], __dmul_rn(pc, __ldg(areas + 3 * (size_t)f + q)));
   }
   const double v = __ldg(V + c);
-  const double vc = v > 1e-30 ? v : 1e-30;
+  const double vc = (__double2hiint(v) >= 0 && above_tiny(v)) ? v : 1e-30;
   const double s = __dmul_rn(alpha, inv_abs_clamped(__ldg(A + c)));
   double u[3];
   for (int q = 0; q < 3; ++q)
-    u[q] = __dsub_rn(__ldg(HbyA + 3 * (size_t)c + q), __dmul_rn(s, __ddiv_rn(g[q], vc)));
-  double m = __dsqrt_rn(__fma_rn(u[2], u[2], __fma_rn(u[1], u[1], __dmul_rn(u[0], u[0]))));
-  m = m > 1e-30 ? m : 1e-30;
-  if (m > 1e4) {
-    const double r = __ddiv_rn(1e4, m);
-    for (int q = 0; q < 3; ++q) u[q] = __dmul_rn(u[q], r);
+    u[q] = __dsub_rn(__ldg(HbyA + 3 * (size_t)c + q), __dmul_rn(s, div_rn(g[q], vc)));
+  const double uu = __fma_rn(u[2], u[2], __fma_rn(u[1], u[1], __dmul_rn(u[0], u[0])));
+  if (above(uu, 1e8)) {  // |U| <= 1e4 otherwise: the root is monotone and exact at 1e8
+    const double m = sqrt_rn(uu);
+    if (above(m, 1e4)) {
+      const double r = div_rn(1e4, m);
+      for (int q = 0; q < 3; ++q) u[q] = __dmul_rn(u[q], r);
+    }
   }
   for (int q = 0; q < 3; ++q) U[3 * (size_t)c + q] = u[q];
 }
@@ -177,7 +198,7 @@ __global__ void __launch_bounds__(kBlock)
     adjust_phi_kernel(int nf, int nint, const double* __restrict__ sum, double* __restrict__ phi) {
   const int f = nint + blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
-  const double corr = __ddiv_rn(*sum, (double)(nf - nint));
+  const double corr = div_rn(*sum, (double)(nf - nint));
   phi[f] = __dsub_rn(phi[f], corr);
 }
 
