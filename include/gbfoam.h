@@ -520,6 +520,18 @@ int gbf_residual_f64(const gbf_layout* L, const double* slot_coef, const double*
  * smooth_solver.py:189-232, smoothers.py:203-260).                         */
 int gbf_relax_f64(int32_t n, double omega, const double* diag, const double* z, double* x,
                   void* stream);
+/* n_sweeps damped Jacobi sweeps x += (omega / max(|diag|, 1e-30)) (b - A x),
+ * each one pass, the bits of gbf_residual_f64 + gbf_relax_f64 (JacobiSmoother,
+ * smoothers.py:152-200; the smoothing of gamg.py:395-420).  scratch[n_cells]
+ * is not x.                                                                 */
+int gbf_jacobi_f64(const gbf_layout* L, const double* slot_coef, const double* diag,
+                   const double* b, double omega, int32_t n_sweeps, double* x, double* scratch,
+                   void* stream);
+/* r = b - A x and *out (DEVICE) = |r|_2: the bits of gbf_residual_f64 +
+ * gbf_norm2_f64; workspace of gbf_norm2_workspace_bytes().                   */
+int gbf_residual_norm2_f64(const gbf_layout* L, const double* slot_coef, const double* diag,
+                           const double* b, const double* x, double* r, double* out,
+                           void* workspace, void* stream);
 /* *out (DEVICE) = |r|_2 in a fixed summation order (the residual norm of
  * solvers/residual.py:112-145); workspace of gbf_norm2_workspace_bytes().  */
 size_t gbf_norm2_workspace_bytes(void);
@@ -548,6 +560,29 @@ int gbf_gamg_coarse_coeffs_f64(int32_t n_cfaces, const int32_t* cf_ptr, const in
                                double* coarse_upper, void* stream);
 int gbf_gamg_prolong_add_f64(int32_t n_fine, const int32_t* f2c, const double* e, double* x,
                              void* stream);
+/* gbf_gamg_restrict_f64 and the coarse correction's start coarse_x = 0.       */
+int gbf_gamg_restrict_start_f64(int32_t n_coarse, const int32_t* agg_ptr, const int32_t* agg_cells,
+                                const double* fine, double* coarse_b, double* coarse_x,
+                                void* stream);
+/* One level of the coarse end of a V-cycle; the transfer arrays lead to the
+ * next level of the array and are unused on the last.                        */
+typedef struct gbf_gamg_level {
+  gbf_layout layout;
+  const double* coef;       /* packed slots (gbf_pack_f64)                     */
+  const double* diag;
+  const int32_t* agg_ptr;   /* fine cells of each aggregate (CSR)              */
+  const int32_t* agg_cells;
+  const int32_t* f2c;
+  int32_t n_coarse, pad;
+} gbf_gamg_level;
+/* The V-cycle from levels_h[0] down to the last level and back in one launch
+ * of one block, with Jacobi smoothing (omega = 1): the bits of the separate
+ * calls.  gbf_gamg_tail_fits tells whether the levels' sizes (host array, fine
+ * first) fit it.                                                             */
+int gbf_gamg_tail_fits(int32_t n_levels, const int32_t* n_cells_h);
+int gbf_gamg_tail_f64(const gbf_gamg_level* levels_h, int32_t n_levels, int32_t n_pre_smooth,
+                      int32_t n_post_smooth, int32_t n_coarsest_sweeps, const double* b, double* x,
+                      void* stream);
 
 /* out = x + a*y (one rounding each; out may alias x or y): the vector
  * updates of PBiCGSolver (solvers/pbicg.py:161-200).                       */

@@ -21,6 +21,7 @@ __all__ = [
     "check",
     "Layout",
     "Batch",
+    "GamgLevel",
     "SolveParams",
     "SolveResult",
     "ptr",
@@ -102,6 +103,21 @@ class Batch(ctypes.Structure):
     ]
 
 
+class GamgLevel(ctypes.Structure):
+    """``gbf_gamg_level``: one level of the coarse end of a V-cycle."""
+
+    _fields_ = [
+        ("layout", Layout),
+        ("coef", _c_vp),
+        ("diag", _c_vp),
+        ("agg_ptr", _c_vp),
+        ("agg_cells", _c_vp),
+        ("f2c", _c_vp),
+        ("n_coarse", _c_i32),
+        ("pad", _c_i32),
+    ]
+
+
 _P = ctypes.POINTER
 _L = _P(Layout)
 
@@ -134,11 +150,20 @@ EXPORTED: dict[str, tuple] = {
     "gbf_gamg_coarse_coeffs_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                                                   _c_vp, _c_vp]),
     "gbf_gamg_prolong_add_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp]),
+    "gbf_gamg_restrict_start_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
+                                                   _c_vp]),
+    "gbf_gamg_tail_fits": (ctypes.c_int, [_c_i32, _P(_c_i32)]),
+    "gbf_gamg_tail_f64": (ctypes.c_int, [_P(GamgLevel), _c_i32, _c_i32, _c_i32, _c_i32, _c_vp,
+                                         _c_vp, _c_vp]),
     "gbf_gs_schedule": (ctypes.c_int, [_c_i32, _c_i32, _c_vp, _c_vp, _c_i32, _c_vp, _c_vp,
                                        _P(_c_i32), _P(_c_i32)]),
     "gbf_gauss_seidel_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32,
                                             _c_dbl, _c_i32, _c_vp, _c_vp, _c_vp]),
     "gbf_residual_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp]),
+    "gbf_jacobi_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_dbl, _c_i32, _c_vp, _c_vp,
+                                      _c_vp]),
+    "gbf_residual_norm2_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
+                                              _c_vp, _c_vp]),
     "gbf_relax_f64": (ctypes.c_int, [_c_i32, _c_dbl, _c_vp, _c_vp, _c_vp, _c_vp]),
     "gbf_norm2_workspace_bytes": (_c_size, []),
     "gbf_norm2_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp]),

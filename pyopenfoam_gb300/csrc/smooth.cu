@@ -20,6 +20,7 @@
 #include <math.h>
 
 #include "amul.cuh"
+#include "exact.cuh"
 #include "wavefront.cuh"
 
 namespace gbf {
@@ -201,15 +202,125 @@ __global__ void gs_flow_out_kernel(int n, const GridBarrier* bar, const double* 
   if (c < n) x[c] = bar->fault != 0 ? __longlong_as_double(0x7ff8000000000000LL) : x_new[c];
 }
 
-// r = b - A x with A x in the reference's order (cell_amul).
-template <int KIND>
+// r_c = b_c - (A x)_c, or with SWEEP one damped Jacobi sweep
+// x_c + (omega / max(|diag_c|, 1e-30)) r_c: residual_kernel's and
+// relax_kernel's operations in their order.
+template <bool SWEEP>
+__device__ __forceinline__ double row_result(double ax, double bc, double dc, double xc,
+                                             double omega) {
+  const double r = __dsub_rn(bc, ax);
+  if (!SWEEP) return r;
+  const double inv = div_rn(1.0, max_abs_tiny(dc));
+  return __dadd_rn(xc, __dmul_rn(omega == 1.0 ? inv : __dmul_rn(omega, inv), r));
+}
+
+// row_result of every cell, a thread per cell: out is not x.  A hex level is
+// bound by the FP64 pipe (16 operations a cell; 262144 cells: residual 8.9 us,
+// sweep 11.3 us, against 8.9 + 1.8 us of a sweep as two kernels with a
+// division per cell in the second).
+template <bool SWEEP>
 __global__ void __launch_bounds__(kBlock)
-    residual_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
-                    const double* __restrict__ b, const double* __restrict__ x,
-                    double* __restrict__ r) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += gridDim.x * blockDim.x)
-    r[c] = __dsub_rn(__ldg(b + c),
-                     cell_amul_k<KIND, double, double, false>(L, coef, diag, x, c, __ldg(x + c)));
+    hex_rows_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
+                    const double* __restrict__ b, double omega, const double* __restrict__ x,
+                    double* __restrict__ out) {
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += gridDim.x * blockDim.x) {
+    const double xc = __ldg(x + c);
+    const double ax =
+        cell_amul_k<kLayoutHex33, double, double, false>(L, coef, diag, x, c, xc);
+    out[c] = row_result<SWEEP>(ax, __ldg(b + c), SWEEP ? __ldg(diag + c) : 1.0, xc, omega);
+  }
+}
+
+// The same on any other layout (coarse multigrid levels, random numberings): a
+// block per 32-cell slice.  A thread per cell walks its row of 10-25 slots
+// through a chain of loads (offset entry, column, x) and of FP64 operations,
+// each of which holds the warp's SM quarter for 64 clocks: 10 us a level
+// however small.  Here the block's warps take the slots in turn (products into
+// shared memory), so all of the slice's loads are in flight together, and then
+// one warp sums the owner side and another the neighbour side in slot order --
+// the products and the order of cell_amul, so its bits: 1148 cells 10.2 -> 3.6
+// us, 8094 cells 9.8 -> 3.8, 32768 cells 10.0 -> 6.6, 131072 cells 15.0 -> 12.8
+// us a sweep.
+// The two summing warps differ from block to block, so that the sums do not
+// all fall on the same quarter of an SM.
+constexpr int kRowSlots = 32;  // slots of a slice held at a time
+
+template <bool SWEEP, int kRowWarps>
+__global__ void __launch_bounds__(32 * kRowWarps)
+    slice_rows_kernel(gbf_layout L, const double* __restrict__ coef,
+                      const double* __restrict__ diag, const double* __restrict__ b, double omega,
+                      const double* __restrict__ x, double* __restrict__ out) {
+  __shared__ double prod[kRowSlots][32];
+  __shared__ unsigned have[kRowSlots];
+  __shared__ double sum_n[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int s = blockIdx.x, c = 32 * s + lane;
+  const unsigned turn = (blockIdx.x * 2654435761u >> 16) & (kRowWarps - 2);
+  const bool owner_sum = warp == (int)turn, neighbour_sum = warp == (int)turn + 1;
+  const CellSlots cs = cell_slots(L, 32 * s + lane);
+  double xc = 0.0, bc = 0.0, dc = 1.0;
+  if (owner_sum && c < L.n_cells) {
+    xc = __ldg(x + c);
+    bc = __ldg(b + c);
+    dc = __ldg(diag + c);
+  }
+  const int W = cs.wo + cs.wn;
+  double sum = 0.0;
+  for (int k0 = 0; k0 < W; k0 += kRowSlots) {
+    const int cnt = W - k0 < kRowSlots ? W - k0 : kRowSlots;
+    int col[kRowSlots / kRowWarps];
+    double a[kRowSlots / kRowWarps];
+#pragma unroll
+    for (int j = 0; j < kRowSlots / kRowWarps; ++j) {
+      const int k = warp + kRowWarps * j;
+      col[j] = k < cnt ? __ldg(L.slot_col + cs.base + 32 * (k0 + k)) : -1;
+      a[j] = k < cnt ? __ldg(coef + cs.base + 32 * (k0 + k)) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kRowSlots / kRowWarps; ++j) {
+      const int k = warp + kRowWarps * j;
+      if (k >= cnt) break;
+      prod[k][lane] = __dmul_rn(a[j], col[j] >= 0 ? __ldg(x + col[j]) : 0.0);
+      const unsigned m = __ballot_sync(0xffffffffu, col[j] >= 0);
+      if (lane == 0) have[k] = m;
+    }
+    __syncthreads();
+    if (owner_sum || neighbour_sum) {
+      const int from = owner_sum ? 0 : (cs.wo > k0 ? cs.wo - k0 : 0);
+      const int to = owner_sum ? (cs.wo - k0 < cnt ? cs.wo - k0 : cnt) : cnt;
+#pragma unroll 4
+      for (int k = from; k < to; ++k) {
+        const double v = __dadd_rn(sum, prod[k][lane]);
+        sum = ((have[k] >> lane) & 1u) ? v : sum;
+      }
+    }
+    __syncthreads();
+  }
+  if (neighbour_sum) sum_n[lane] = sum;
+  __syncthreads();
+  if (owner_sum && c < L.n_cells) {
+    double ax = __dmul_rn(dc, xc);
+    if (L.n_faces > 0) ax = __dadd_rn(__dadd_rn(ax, sum), sum_n[lane]);
+    out[c] = row_result<SWEEP>(ax, bc, dc, xc, omega);
+  }
+}
+
+// Slices that eight warps each keep resident at once (8 blocks on 152 SMs);
+// above, four warps a slice.
+constexpr int kRowFewSlices = 8 * 152;
+
+template <bool SWEEP>
+static void launch_rows(const gbf_layout* L, const double* coef, const double* diag,
+                        const double* b, double omega, const double* x, double* out,
+                        cudaStream_t s) {
+  if (layout_kind(*L) == kLayoutHex33) {
+    const int grid = wave_grid(hex_rows_kernel<SWEEP>, kBlock, L->n_cells);
+    hex_rows_kernel<SWEEP><<<grid, kBlock, 0, s>>>(*L, coef, diag, b, omega, x, out);
+  } else if (L->n_slices <= kRowFewSlices) {
+    slice_rows_kernel<SWEEP, 8><<<L->n_slices, 256, 0, s>>>(*L, coef, diag, b, omega, x, out);
+  } else {
+    slice_rows_kernel<SWEEP, 4><<<L->n_slices, 128, 0, s>>>(*L, coef, diag, b, omega, x, out);
+  }
 }
 
 // x += (omega * s_c) * z with s_c = 1 / max(|diag_c|, 1e-30), or
@@ -221,8 +332,7 @@ __global__ void __launch_bounds__(kBlock)
   if (c >= n) return;
   double s = omega;
   if (diag) {
-    const double a = fabs(__ldg(diag + c));
-    s = __dmul_rn(omega, __ddiv_rn(1.0, a > 1e-30 ? a : 1e-30));
+    s = __dmul_rn(omega, div_rn(1.0, max_abs_tiny(__ldg(diag + c))));
   }
   x[c] = __dadd_rn(x[c], __dmul_rn(s, __ldg(z + c)));
 }
@@ -286,6 +396,26 @@ __global__ void __launch_bounds__(kBlock)
   double s = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     const double v = __ldg(r + c);
+    s = __fma_rn(v, v, s);
+  }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+}
+
+// r = b - A x and the per-block sums of r^2 in one pass, over the cells and in
+// the order of sumsq_partials_kernel.
+template <int KIND>
+__global__ void __launch_bounds__(kBlock)
+    residual_sumsq_kernel(gbf_layout L, const double* __restrict__ coef,
+                          const double* __restrict__ diag, const double* __restrict__ b,
+                          const double* __restrict__ x, double* __restrict__ r,
+                          double* __restrict__ partials) {
+  __shared__ double sh[kBlock / 32];
+  double s = 0.0;
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += gridDim.x * blockDim.x) {
+    const double v = __dsub_rn(
+        __ldg(b + c), cell_amul_k<KIND, double, double, false>(L, coef, diag, x, c, __ldg(x + c)));
+    r[c] = v;
     s = __fma_rn(v, v, s);
   }
   s = block_sum(s, sh);
@@ -388,13 +518,51 @@ extern "C" int gbf_residual_f64(const gbf_layout* L, const double* coef, const d
   if (L->n_cells == 0) return GBF_OK;
   GBF_REQUIRE(diag && b && x && r && (L->n_faces == 0 || coef), "residual: NULL pointer");
   cudaStream_t s = as_stream(stream);
-  if (layout_kind(*L) == kLayoutHex33) {
-    const int grid = wave_grid(residual_kernel<kLayoutHex33>, kBlock, L->n_cells);
-    residual_kernel<kLayoutHex33><<<grid, kBlock, 0, s>>>(*L, coef, diag, b, x, r);
-  } else {
-    const int grid = wave_grid(residual_kernel<kLayoutGeneric>, kBlock, L->n_cells);
-    residual_kernel<kLayoutGeneric><<<grid, kBlock, 0, s>>>(*L, coef, diag, b, x, r);
+  launch_rows<false>(L, coef, diag, b, 1.0, x, r, s);
+  GBF_CHECK_LAUNCH();
+  return GBF_OK;
+}
+
+extern "C" int gbf_jacobi_f64(const gbf_layout* L, const double* coef, const double* diag,
+                              const double* b, double omega, int32_t n_sweeps, double* x,
+                              double* scratch, void* stream) {
+  int rc = check_layout(L);
+  if (rc) return rc;
+  GBF_REQUIRE(n_sweeps >= 0, "jacobi: negative n_sweeps");
+  if (L->n_cells == 0 || n_sweeps == 0) return GBF_OK;
+  GBF_REQUIRE(diag && b && x && scratch && scratch != x && (L->n_faces == 0 || coef),
+              "jacobi: NULL pointer, or scratch is x");
+  cudaStream_t s = as_stream(stream);
+  double *from = x, *to = scratch;
+  for (int k = 0; k < n_sweeps; ++k) {
+    launch_rows<true>(L, coef, diag, b, omega, from, to, s);
+    double* t = from;
+    from = to;
+    to = t;
   }
+  GBF_CHECK_LAUNCH();
+  if (from != x)  // an odd number of sweeps ends in the scratch
+    GBF_CHECK_CUDA(cudaMemcpyAsync(x, from, sizeof(double) * (size_t)L->n_cells,
+                                   cudaMemcpyDeviceToDevice, s));
+  return GBF_OK;
+}
+
+extern "C" int gbf_residual_norm2_f64(const gbf_layout* L, const double* coef, const double* diag,
+                                      const double* b, const double* x, double* r, double* out,
+                                      void* workspace, void* stream) {
+  int rc = check_layout(L);
+  if (rc) return rc;
+  const int n = L->n_cells;
+  GBF_REQUIRE(out && workspace && (n == 0 || (diag && b && x && r)) && (L->n_faces == 0 || coef),
+              "residual_norm2: NULL pointer");
+  cudaStream_t s = as_stream(stream);
+  int g = (n + kBlock - 1) / kBlock;
+  g = g < 1 ? 1 : (g > kNormBlocks ? kNormBlocks : g);
+  double* partials = static_cast<double*>(workspace);
+  GBF_LAYOUT_DISPATCH(*L, K, residual_sumsq_kernel<K><<<g, kBlock, 0, s>>>(*L, coef, diag, b, x, r,
+                                                                           partials));
+  GBF_CHECK_LAUNCH();
+  sqrt_sum_kernel<<<1, kBlock, 0, s>>>(g, partials, out);
   GBF_CHECK_LAUNCH();
   return GBF_OK;
 }

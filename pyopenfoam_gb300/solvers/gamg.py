@@ -36,7 +36,7 @@ from .. import _lib
 from ..core.ldu_matrix import LduMatrix
 from .linear_solver import LinearSolverBase
 from .residual import ConvergenceInfo, ResidualMonitor
-from .smoothers import relax, residual
+from .smoothers import residual
 
 __all__ = ["GAMGSolver", "GAMGLevel", "AggregationData"]
 
@@ -207,15 +207,47 @@ class GAMGSolver(LinearSolverBase):
         matrix._csr_cache[key] = out
         return out
 
+    def _tail(self, levels, aggs):
+        """(first level, descriptors) of the coarse end that one launch takes
+        (``gbf_gamg_tail_f64``); (len(levels), None) when not even the coarsest
+        level fits."""
+        L = _lib.lib()
+        first = len(levels)
+        while first > 0:
+            sizes = [lv.n_cells for lv in levels[first - 1:]]
+            if not L.gbf_gamg_tail_fits(len(sizes), (ctypes.c_int32 * len(sizes))(*sizes)):
+                break
+            first -= 1
+        if first == len(levels):
+            return first, None
+        desc = (_lib.GamgLevel * (len(levels) - first))()
+        for k, lv in enumerate(levels[first:]):
+            m, d = lv.matrix, desc[k]
+            d.layout = m.topology().layout
+            d.coef, d.diag = m.packed().data_ptr(), m.diag.data_ptr()
+            if first + k < len(aggs):
+                agg = aggs[first + k]
+                d.agg_ptr, d.agg_cells = agg.agg_ptr.data_ptr(), agg.agg_cells.data_ptr()
+                d.f2c, d.n_coarse = agg.f2c32.data_ptr(), agg.n_coarse
+        return first, desc
+
     @staticmethod
     def _jacobi(m: LduMatrix, x: torch.Tensor, b: torch.Tensor, n_it: int,
                 r: torch.Tensor) -> None:
-        for _ in range(n_it):
-            residual(m, b, x, r)
-            relax(x, r, 1.0, m.diag)
+        _lib.check(_lib.lib().gbf_jacobi_f64(
+            m.topology().layout_ref, m.packed().data_ptr(), m.diag.data_ptr(), b.data_ptr(), 1.0,
+            int(n_it), x.data_ptr(), r.data_ptr(), _lib.stream_ptr(m.device)), "gbf_jacobi_f64")
 
-    def _v_cycle(self, levels, aggs, i: int, x: torch.Tensor, b: torch.Tensor) -> None:
+    def _v_cycle(self, levels, aggs, i: int, x: torch.Tensor, b: torch.Tensor, tail) -> None:
         m = levels[i].matrix
+        st = _lib.stream_ptr(m.device)
+        L = _lib.lib()
+        first, desc = tail
+        if i == first:
+            _lib.check(L.gbf_gamg_tail_f64(desc, len(desc), self._n_pre_smooth,
+                                           self._n_post_smooth, 50, b.data_ptr(), x.data_ptr(),
+                                           st), "gbf_gamg_tail_f64")
+            return
         r = torch.empty_like(x)
         if i == len(levels) - 1:
             self._jacobi(m, x, b, 50, r)
@@ -223,14 +255,13 @@ class GAMGSolver(LinearSolverBase):
         self._jacobi(m, x, b, self._n_pre_smooth, r)
         residual(m, b, x, r)
         agg = aggs[i]
-        st = _lib.stream_ptr(m.device)
-        L = _lib.lib()
         rc = torch.empty(agg.n_coarse, device=m.device, dtype=torch.float64)
-        _lib.check(L.gbf_gamg_restrict_f64(agg.n_coarse, agg.agg_ptr.data_ptr(),
-                                           agg.agg_cells.data_ptr(), r.data_ptr(), rc.data_ptr(),
-                                           st), "gbf_gamg_restrict_f64")
-        ec = torch.zeros_like(rc)
-        self._v_cycle(levels, aggs, i + 1, ec, rc)
+        ec = torch.empty_like(rc)
+        _lib.check(L.gbf_gamg_restrict_start_f64(agg.n_coarse, agg.agg_ptr.data_ptr(),
+                                                 agg.agg_cells.data_ptr(), r.data_ptr(),
+                                                 rc.data_ptr(), ec.data_ptr(), st),
+                   "gbf_gamg_restrict_start_f64")
+        self._v_cycle(levels, aggs, i + 1, ec, rc, tail)
         _lib.check(L.gbf_gamg_prolong_add_f64(m.n_cells, agg.f2c32.data_ptr(), ec.data_ptr(),
                                               x.data_ptr(), st), "gbf_gamg_prolong_add_f64")
         self._jacobi(m, x, b, self._n_post_smooth, r)
@@ -259,7 +290,7 @@ class GAMGSolver(LinearSolverBase):
 
     def _cycle(self, matrix: LduMatrix, levels, aggs) -> dict:
         """One V-cycle plus the residual norm on static buffers, captured
-        once into a CUDA graph per hierarchy (the cycle is a few hundred
+        once into a CUDA graph per hierarchy (the cycle is a few dozen
         small launches, so replaying the graph removes the per-launch host
         cost); eager launches if capture is off or fails."""
         key = ("gamg_cycle", id(levels))
@@ -275,12 +306,15 @@ class GAMGSolver(LinearSolverBase):
                                  dtype=torch.uint8),
                "nrm": torch.empty(1, device=dev, dtype=torch.float64), "levels": levels}
 
+        tail = self._tail(levels, aggs)
+
         def body():
-            self._v_cycle(levels, aggs, 0, buf["x"], buf["b"])
-            residual(matrix, buf["b"], buf["x"], buf["r"])
-            _lib.check(L.gbf_norm2_f64(n, buf["r"].data_ptr(), buf["nrm"].data_ptr(),
-                                       buf["ws"].data_ptr(), _lib.stream_ptr(dev)),
-                       "gbf_norm2_f64")
+            self._v_cycle(levels, aggs, 0, buf["x"], buf["b"], tail)
+            _lib.check(L.gbf_residual_norm2_f64(
+                matrix.topology().layout_ref, matrix.packed().data_ptr(), matrix.diag.data_ptr(),
+                buf["b"].data_ptr(), buf["x"].data_ptr(), buf["r"].data_ptr(),
+                buf["nrm"].data_ptr(), buf["ws"].data_ptr(), _lib.stream_ptr(dev)),
+                "gbf_residual_norm2_f64")
 
         buf["run"] = body
         if self._use_graph and n > 0:

@@ -150,10 +150,12 @@ class JacobiSmoother:
         m = self._matrix
         x = _f64(m, x, "x").clone()
         b = _f64(m, b, "b")
-        r = torch.empty_like(x)
-        for _ in range(n_iterations):
-            residual(m, b, x, r)
-            relax(x, r, self._omega, m.diag)
+        if n_iterations > 0:
+            r = torch.empty_like(x)
+            _lib.check(_lib.lib().gbf_jacobi_f64(
+                m.topology().layout_ref, m.packed().data_ptr(), m.diag.data_ptr(), b.data_ptr(),
+                float(self._omega), int(n_iterations), x.data_ptr(), r.data_ptr(),
+                _lib.stream_ptr(m.device)), "gbf_jacobi_f64")
         return x
 
 
