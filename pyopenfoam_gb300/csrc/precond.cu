@@ -3,6 +3,7 @@
 #include <math.h>
 #include <string.h>
 
+#include "exact.cuh"
 #include "wavefront.cuh"
 
 namespace gbf {
@@ -157,8 +158,11 @@ __global__ void __launch_bounds__(kBlock)
 // (every cell's factored value is written once, by its own step, and read
 // only by cells after it).  The subtractions of dic_cell, in slot order: a
 // pass first issues the loads of every slot still pending (they are
-// independent, so their round trips overlap), then applies the slots in
-// order up to the first one still empty.  Cells with more than four
+// independent, so their round trips overlap), forms the quotient of each that
+// has arrived, then subtracts the quotients in order up to the first one still
+// empty.  The chain from level to level is what bounds the walk, so a*a is
+// formed before the wait and the divisions run on the integer pipe (303 clocks
+// against 560, and several at once).  Cells with more than four
 // neighbour-side slots (polyhedral meshes) walk them one load at a time.
 __global__ void __launch_bounds__(kBlock)
     dic_flow_kernel(gbf_layout L, const double* __restrict__ coef,
@@ -176,7 +180,8 @@ __global__ void __launch_bounds__(kBlock)
     int c = 0, k = 0, wn = 0, base = 0;
     double dc = 0.0;
     int j[4] = {-1, -1, -1, -1};
-    double a[4] = {0.0, 0.0, 0.0, 0.0}, dv[4] = {0.0, 0.0, 0.0, 0.0};
+    double a[4] = {0.0, 0.0, 0.0, 0.0};  // a * a, then the quotient
+    unsigned wait = 0, take = 0;         // slots still empty; slots with a quotient
     if (!done) {
       c = __ldg(cells + i);
       dc = __ldg(diag + c);
@@ -186,12 +191,25 @@ __global__ void __launch_bounds__(kBlock)
         base = cs.base + 32 * cs.wo;
       }
       if (wn <= 4) {
+        double dv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           if (q < wn) {
             j[q] = __ldg(L.slot_col + base + 32 * q);
             a[q] = __ldg(coef + base + 32 * q);
-            if (j[q] > c) dv[q] = __ldg(diag + j[q]);  // unfactored: read once
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dv[q] = j[q] > c ? __ldg(diag + j[q]) : 0.0;  // unfactored
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if (j[q] < 0) continue;
+          a[q] = __dmul_rn(a[q], a[q]);
+          if (j[q] < c) {
+            wait |= 1u << q;
+          } else if (above_tiny(fabs(dv[q]))) {
+            a[q] = div_rn(a[q], dv[q]);
+            take |= 1u << q;
           }
         }
       }
@@ -200,18 +218,26 @@ __global__ void __launch_bounds__(kBlock)
     for (;;) {
       if (!done) {
         if (wn <= 4) {
+          if (wait) {
+            double v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) v[q] = (wait >> q & 1u) ? ld_flow(d + j[q]) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if ((wait >> q & 1u) && !flow_empty(v[q])) {
+                wait &= ~(1u << q);
+                if (above_tiny(fabs(v[q]))) {
+                  a[q] = div_rn(a[q], v[q]);
+                  take |= 1u << q;
+                }
+              }
+          }
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            if (q >= k && j[q] >= 0 && j[q] < c) dv[q] = ld_flow(d + j[q]);
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            if (q == k && q < wn) {
-              if (j[q] >= 0 && j[q] < c && flow_empty(dv[q])) continue;  // stays at k
-              if (j[q] >= 0 && fabs(dv[q]) > 1e-30)
-                dc = __dsub_rn(dc, __ddiv_rn(__dmul_rn(a[q], a[q]), dv[q]));
+            if (k == q && q < wn && !(wait >> q & 1u)) {
+              if (take >> q & 1u) dc = __dsub_rn(dc, a[q]);
               k = q + 1;
             }
-          }
         } else {
           for (; k < wn; ++k) {
             const int s = base + 32 * k;
@@ -224,9 +250,9 @@ __global__ void __launch_bounds__(kBlock)
             } else {
               dj = __ldg(diag + jk);
             }
-            if (fabs(dj) > 1e-30) {
+            if (above_tiny(fabs(dj))) {
               const double ak = __ldg(coef + s);
-              dc = __dsub_rn(dc, __ddiv_rn(__dmul_rn(ak, ak), dj));
+              dc = __dsub_rn(dc, div_rn(__dmul_rn(ak, ak), dj));
             }
           }
         }
@@ -261,11 +287,10 @@ __global__ void __launch_bounds__(kBlock)
     const long long i = ch * 32 + lane;
     bool done = i >= nf;
     int sp = -1, sq = -1;
-    double a = 0.0, b = 0.0, l = 0.0, u = 0.0;
+    double a = 0.0, b = 0.0, lu = 0.0;
     if (!done) {
       const int f = __ldg(faces + i);
-      l = __ldg(lower + f);
-      u = __ldg(upper + f);
+      lu = __dmul_rn(__ldg(lower + f), __ldg(upper + f));  // = upper * lower
       sp = __ldg(prev + 2 * i);
       sq = __ldg(prev + 2 * i + 1);
       if (sp < 0) a = __ldg(diag + __ldg(L.owner + f));
@@ -287,8 +312,8 @@ __global__ void __launch_bounds__(kBlock)
         }
         if (sp < 0 && sq < 0) {
           double na = a, nb = b;
-          if (fabs(b) > 1e-30) na = __dsub_rn(a, __ddiv_rn(__dmul_rn(l, u), b));
-          if (fabs(a) > 1e-30) nb = __dsub_rn(b, __ddiv_rn(__dmul_rn(u, l), a));
+          if (above_tiny(fabs(b))) na = __dsub_rn(a, div_rn(lu, b));
+          if (above_tiny(fabs(a))) nb = __dsub_rn(b, div_rn(lu, a));
           st_flow(slots + 2 * i, na);
           st_flow(slots + 2 * i + 1, nb);
           done = true;
@@ -343,7 +368,7 @@ __global__ void copy_kernel(int n, const double* __restrict__ s, double* __restr
 __global__ void diag_apply_kernel(int n, const double* __restrict__ r,
                                   const double* __restrict__ d, double* __restrict__ z) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < n) z[c] = __ddiv_rn(r[c], d[c]);
+  if (c < n) z[c] = div_rn(r[c], d[c]);
 }
 
 }  // namespace gbf
@@ -683,7 +708,7 @@ __global__ void __launch_bounds__(kBlock)
         }
         if (sw < 0 && sr < 0) {
           st_flow(slots + i,
-                  fabs(dr) > 1e-30 ? __dsub_rn(w, __ddiv_rn(__dmul_rn(cf, r), dr)) : w);
+                  above_tiny(fabs(dr)) ? __dsub_rn(w, div_rn(__dmul_rn(cf, r), dr)) : w);
           done = true;
         }
       }

@@ -96,11 +96,11 @@ __device__ __forceinline__ double gs_row(const gbf_layout& L, const double* __re
 // The updated value of cell c from its row sum (the value itself when the
 // diagonal is too small to divide by, as in the reference).
 template <bool RELAX>
-__device__ __forceinline__ double gs_update(double row, double dc, double xc, double bc,
+__device__ __forceinline__ double gs_update(double row, double dx, double dc, double xc, double bc,
                                             double omega) {
-  const double off = __dsub_rn(row, __dmul_rn(dc, xc));
-  if (!(fabs(dc) > 1e-30)) return xc;
-  const double nv = __ddiv_rn(__dsub_rn(bc, off), dc);
+  const double off = __dsub_rn(row, dx);  // dx = dc * xc, rounded
+  if (!above_tiny(fabs(dc))) return xc;
+  const double nv = div_rn(__dsub_rn(bc, off), dc);
   return RELAX ? __dadd_rn(xc, __dmul_rn(omega, __dsub_rn(nv, xc))) : nv;
 }
 
@@ -112,7 +112,8 @@ __device__ __forceinline__ void gs_cell(const gbf_layout& L, const double* __res
   const double dc = __ldg(diag + c);
   const double xc = __ldcg(x + c);
   const double row = gs_row(L, coef, dc, xc, c, [&](int col) { return __ldcg(x + col); });
-  if (fabs(dc) > 1e-30) x[c] = gs_update<RELAX>(row, dc, xc, __ldg(b + c), omega);
+  if (above_tiny(fabs(dc)))
+    x[c] = gs_update<RELAX>(row, __dmul_rn(dc, xc), dc, xc, __ldg(b + c), omega);
 }
 
 template <bool RELAX>
@@ -147,8 +148,19 @@ __global__ void __launch_bounds__(kBlock)
 // x_new (initialised to the empty marker); a cell polls only the new values
 // it reads -- its neighbours swept before it (lower-numbered forward,
 // higher-numbered backward), which are at earlier levels -- so the warp
-// holding the earliest unfinished cell always finds its inputs.  The row sum
-// and the update are gs_cell's (gs_row, gs_update): the same bits.
+// holding the earliest unfinished cell always finds its inputs.
+//
+// What bounds it is the chain from one level to the next: the store, its
+// neighbour's poll, and the FP64 operations between them, 64 clocks each (a
+// CUDA divide 560).  So everything that does not need a new value happens
+// before the wait -- loads, the products with old values, the sum up to the
+// first new value -- a pass only polls what is still missing, and an arrival
+// costs its product, the rest of the row's additions and one integer-pipe
+// division.  Repeating gs_row on every pass instead took 5.1 us a level
+// (67 x 59 x 53 cells: 902 us a sweep, 466 us now).  The products, their order
+// and the update are gs_cell's (gs_row, gs_update): the same bits.  Cells with
+// more than four slots a side, and cells whose owner-side faces do not all
+// follow their neighbour-side faces, repeat gs_row.
 template <bool RELAX>
 __global__ void __launch_bounds__(kBlock)
     gs_flow_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
@@ -166,26 +178,87 @@ __global__ void __launch_bounds__(kBlock)
     bool done = i >= n;
     int c = 0;
     double dc = 0.0, xc = 0.0, bc = 0.0;
+    // slots in face order: position o is neighbour-side slot o (o < 4), then
+    // owner-side slot o - 4
+    bool ordered = false;
+    unsigned used = 0, wait = 0;  // positions with a face; with a new value still to come
+    int q[8];
+    double p[8], row = 0.0, dx = 0.0;  // p: the product, or the coefficient while waiting
+    int pos = 0;
     if (!done) {
       c = __ldg(cells + i);
       dc = __ldg(diag + c);
       xc = __ldg(x_old + c);
       bc = __ldg(b + c);
+      if (L.n_faces > 0) {
+        const CellSlots cs = cell_slots(L, c);
+        if (cs.wo <= 4 && cs.wn <= 4) {
+          int max_nei = -1, min_own = INT_MAX;
+#pragma unroll
+          for (int o = 0; o < 8; ++o) {
+            const bool use = o < 4 ? o < cs.wn : o - 4 < cs.wo;
+            const int k = o < 4 ? cs.wo + o : o - 4;
+            const int slot = cs.base + 32 * k;
+            const int f = use ? __ldg(L.slot_face + slot) : -1;
+            q[o] = use ? slot_column(L, cs.e0 + k, slot, c) : -1;
+            p[o] = use ? __ldg(coef + slot) : 0.0;
+            if (f >= 0 && q[o] >= 0) {
+              used |= 1u << o;
+              if (reverse ? q[o] > c : q[o] < c) wait |= 1u << o;
+              if (o < 4) max_nei = f;
+              else if (min_own == INT_MAX) min_own = f;
+            }
+          }
+          ordered = max_nei < min_own;
+          if (ordered) {
+            double v[8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o)
+              v[o] = ((used & ~wait) >> o & 1u) ? __ldg(x_old + q[o]) : 0.0;
+#pragma unroll
+            for (int o = 0; o < 8; ++o)
+              if ((used & ~wait) >> o & 1u) p[o] = __dmul_rn(p[o], v[o]);
+          }
+        }
+      }
+      dx = __dmul_rn(dc, xc);
+      row = dx;
     }
     bool quit = false;
     for (;;) {
       if (!done) {
         bool missing = false;
-        const double row = gs_row(L, coef, dc, xc, c, [&](int col) {
-          if (reverse ? col > c : col < c) {
-            const double v = ld_flow(x_new + col);
-            missing |= flow_empty(v);
-            return v;
+        if (ordered) {
+          if (wait) {
+            double v[8];
+#pragma unroll
+            for (int o = 0; o < 8; ++o) v[o] = (wait >> o & 1u) ? ld_flow(x_new + q[o]) : 0.0;
+#pragma unroll
+            for (int o = 0; o < 8; ++o)
+              if ((wait >> o & 1u) && !flow_empty(v[o])) {
+                p[o] = __dmul_rn(p[o], v[o]);
+                wait &= ~(1u << o);
+              }
           }
-          return __ldg(x_old + col);
-        });
+#pragma unroll
+          for (int o = 0; o < 8; ++o)
+            if (pos == o && !(wait >> o & 1u)) {
+              if (used >> o & 1u) row = __dadd_rn(row, p[o]);
+              pos = o + 1;
+            }
+          missing = pos < 8;
+        } else {
+          row = gs_row(L, coef, dc, xc, c, [&](int col) {
+            if (reverse ? col > c : col < c) {
+              const double v = ld_flow(x_new + col);
+              missing |= flow_empty(v);
+              return v;
+            }
+            return __ldg(x_old + col);
+          });
+        }
         if (!missing) {
-          st_flow(x_new + c, gs_update<RELAX>(row, dc, xc, bc, omega));
+          st_flow(x_new + c, gs_update<RELAX>(row, dx, dc, xc, bc, omega));
           done = true;
         }
       }
