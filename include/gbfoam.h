@@ -302,6 +302,11 @@ int gbf_dilu_build_f64(const gbf_layout* L, const double* lower, const double* u
 int gbf_dic_build_flow_f64(const gbf_layout* L, const double* coef, const double* diag,
                            const int32_t* level_cells, double* d_out, void* barrier,
                            void* stream);
+/* DIC with the cells dealt to blocks, as gbf_gauss_seidel_block_f64.          */
+int gbf_dic_build_block_f64(const gbf_layout* L, const double* coef, const double* diag,
+                            const int32_t* block_cells, const int32_t* block_ptr,
+                            int32_t n_blocks, int32_t per, double* d_out, void* barrier,
+                            void* stream);
 /* DILU (preconditioners.py:228-272): the faces of gbf_dilu_schedule in level
  * order with the links of gbf_dilu_flow_links; slots = device scratch of
  * gbf_dilu_flow_slots_bytes(n_faces) bytes.                                */
@@ -511,6 +516,16 @@ int gbf_gauss_seidel_flow_f64(const gbf_layout* L, const double* coef, const dou
                               const double* b, const int32_t* level_cells, int32_t reverse,
                               double omega, int32_t relax, double* x, double* scratch,
                               void* barrier, void* stream);
+/* The same walk with the cells dealt to blocks: block b of n_blocks takes the
+ * cells [b per, (b+1) per), listed in level order at block_cells[block_ptr[b]]
+ * on, and passes values between its own cells through shared memory.  All
+ * n_blocks must be resident at once (one per SM); per <= 24576; a cell index
+ * listed under block b lies in its range.                                    */
+int gbf_gauss_seidel_block_f64(const gbf_layout* L, const double* slot_coef, const double* diag,
+                               const double* b, const int32_t* block_cells,
+                               const int32_t* block_ptr, int32_t n_blocks, int32_t per,
+                               int32_t reverse, double omega, int32_t relax, double* x,
+                               double* scratch, void* barrier, void* stream);
 /* r = b - A x, A x bitwise LduMatrix.Ax (core/ldu_matrix.py:172-217); the
  * residual of every smoother and of the smoothing solvers.                 */
 int gbf_residual_f64(const gbf_layout* L, const double* slot_coef, const double* diag,

@@ -232,6 +232,11 @@ EXPORTED: dict[str, tuple] = {
                                           _c_vp, _c_vp, _c_vp]),
     "gbf_gauss_seidel_flow_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32, _c_dbl,
                                                  _c_i32, _c_vp, _c_vp, _c_vp, _c_vp]),
+    "gbf_gauss_seidel_block_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32,
+                                                  _c_i32, _c_i32, _c_dbl, _c_i32, _c_vp, _c_vp,
+                                                  _c_vp, _c_vp]),
+    "gbf_dic_build_block_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32, _c_i32,
+                                               _c_vp, _c_vp, _c_vp]),
     "gbf_sweep_flow_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_i32, _c_vp, _c_vp, _c_i32,
                                           _c_vp, _c_vp, _c_vp, _c_vp]),
     "gbf_dic_build_flow_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp]),

@@ -43,6 +43,42 @@ class FlowLinks:
     cell_last: torch.Tensor
 
 
+@dataclass
+class BlockOrder:
+    """Cells of a level schedule dealt to resident blocks: block b takes the
+    cells [b * per, (b + 1) * per), in level order at cells[ptr[b]:ptr[b + 1]]."""
+
+    ptr: torch.Tensor
+    cells: torch.Tensor
+    n_blocks: int
+    per: int
+
+
+#: Cells a block of a block walk may keep in shared memory (8 bytes each; a
+#: larger system, 3.7 million cells on 152 SMs, runs the walk over the whole
+#: schedule).  A block takes at least the smaller number, so that most links
+#: between neighbouring cells stay inside it.
+WALK_CELLS_MAX = 24576
+WALK_CELLS_MIN = 512
+
+
+def block_order(level_cells: np.ndarray, device: torch.device) -> BlockOrder | None:
+    """The block order of a schedule's cells, or None when a block per SM
+    cannot keep its share of them."""
+    n = level_cells.shape[0]
+    sms = torch.cuda.get_device_properties(device).multi_processor_count
+    per = max(WALK_CELLS_MIN, -(-n // sms))
+    if n == 0 or per > WALK_CELLS_MAX:
+        return None
+    block = level_cells // per
+    n_blocks = -(-n // per)
+    cells = level_cells[np.argsort(block.astype(np.uint16), kind="stable")]
+    ptr = np.zeros(n_blocks + 1, np.int32)
+    np.cumsum(np.bincount(block, minlength=n_blocks), out=ptr[1:])
+    return BlockOrder(torch.from_numpy(ptr).to(device),
+                      torch.from_numpy(np.ascontiguousarray(cells)).to(device), n_blocks, per)
+
+
 def _i32_host(t: torch.Tensor, n_cells: int, name: str) -> np.ndarray:
     a = t.detach().to("cpu", torch.int64).numpy()
     if a.size and (a.min() < 0 or a.max() >= n_cells):
@@ -182,7 +218,13 @@ class Topology:
             )
             self._dic = Schedule(torch.from_numpy(ptr[: nl.value + 1].copy()).to(self.device),
                                  torch.from_numpy(cells).to(self.device), nl.value, mx.value)
+            self._dic_blocks = block_order(cells[:n], self.device)
         return self._dic
+
+    def dic_blocks(self) -> BlockOrder | None:
+        """``dic_schedule()``'s cells dealt to blocks (see ``block_order``)."""
+        self.dic_schedule()
+        return self._dic_blocks
 
     def dilu_schedule(self) -> Schedule:
         if self._dilu is None:

@@ -59,39 +59,75 @@ __device__ __forceinline__ uint32_t fix22(float y) {
   return __float_as_uint(__fmaf_rn(y, 4194304.0f, 8388608.0f)) - 0x4b000000u;
 }
 
+// A division under way: the operands' words, mantissas and exponents and the
+// quotient's digits.
+struct DivDigits {
+  uint32_t ah, bh, ea, eb;
+  uint64_t ma, mb, q;  // q: mantissa quotient at 2^-63, within 2 units
+  uint32_t up, half;   // up 1: quotient in [1, 2), 0: in (1/2, 1); half a result ulp of q
+
+  __device__ __forceinline__ DivDigits(double a, double b) {
+    ah = (uint32_t)__double2hiint(a);
+    bh = (uint32_t)__double2hiint(b);
+    const uint32_t al = (uint32_t)__double2loint(a), bl = (uint32_t)__double2loint(b);
+    ea = (ah >> 20) & 0x7ffu;
+    eb = (bh >> 20) & 0x7ffu;
+    const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
+    ma = ((uint64_t)mah << 32) | al;
+    mb = ((uint64_t)mbh << 32) | bl;
+    // fa, fb in [1, 2): the mantissas' top 24 bits; quotient digits Q0 at
+    // 2^-22, Q1 at 2^-48, q at 2^-63
+    const float fa = __uint_as_float(__funnelshift_l(al, mah, 3) + 0x3f000000u);
+    const float fb = __uint_as_float(__funnelshift_l(bl, mbh, 3) + 0x3f000000u);
+    const float y = rcp_approx(fb);
+    const int Y = (int)(fix22(y) << 8);
+    const uint32_t Q0 = fix22(__fmul_rn(fa, y));
+    const int64_t r0 = (int64_t)((ma << 22) - (uint64_t)Q0 * mb);
+    const int D1 = __mulhi((int)(r0 >> 24), Y);
+    const uint64_t Q1 = ((uint64_t)Q0 << 26) + (int64_t)D1;
+    const int64_t r1 = (int64_t)((ma << 48) - Q1 * mb);
+    const int D2 = __mulhi((int)(r1 >> 29), Y);
+    q = (Q1 << 15) + (int64_t)(D2 >> 6);
+    up = (uint32_t)(q >> 63);
+    half = 512u << up;
+  }
+  // both operands and the quotient well inside the normal range
+  __device__ __forceinline__ bool normal() const {
+    return ea - 1u < 2046u && eb - 1u < 2046u && ea - eb + 1000u <= 2000u;
+  }
+  // within 3 units of a midpoint between two results
+  __device__ __forceinline__ bool close() const {
+    return (((uint32_t)q + half + 3u) & (2u * half - 1u)) < 6u;
+  }
+  __device__ __forceinline__ uint64_t rounded() const { return (q + half) >> (10 + up); }
+  __device__ __forceinline__ double result(uint64_t m) const {
+    const uint32_t ex = ea - eb + 1021u + up;
+    const uint32_t hi = ((uint32_t)(m >> 32) + (ex << 20)) | ((ah ^ bh) & 0x80000000u);
+    return __hiloint2double((int)hi, (int)(uint32_t)m);
+  }
+};
+
 // a / b, the bits of __ddiv_rn.
 __device__ __forceinline__ double div_rn(double a, double b) {
-  const uint32_t ah = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
-  const uint32_t bh = (uint32_t)__double2hiint(b), bl = (uint32_t)__double2loint(b);
-  const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (bh >> 20) & 0x7ffu;
-  if (ea - 1u >= 2046u || eb - 1u >= 2046u || ea - eb + 1000u > 2000u) return div_rn_slow(a, b);
-  const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
-  const uint64_t ma = ((uint64_t)mah << 32) | al, mb = ((uint64_t)mbh << 32) | bl;
-  const float fa = __uint_as_float(__funnelshift_l(al, mah, 3) + 0x3f000000u);
-  const float fb = __uint_as_float(__funnelshift_l(bl, mbh, 3) + 0x3f000000u);
-  const float y = rcp_approx(fb);
-  const int Y = (int)(fix22(y) << 8);
-  // fa, fb in [1, 2): the mantissas' top 24 bits; quotient digits Q0 at
-  // 2^-22, Q1 at 2^-48, q at 2^-63
-  const uint32_t Q0 = fix22(__fmul_rn(fa, y));
-  const int64_t r0 = (int64_t)((ma << 22) - (uint64_t)Q0 * mb);
-  const int D1 = __mulhi((int)(r0 >> 24), Y);
-  const uint64_t Q1 = ((uint64_t)Q0 << 26) + (int64_t)D1;
-  const int64_t r1 = (int64_t)((ma << 48) - Q1 * mb);
-  const int D2 = __mulhi((int)(r1 >> 29), Y);
-  const uint64_t q = (Q1 << 15) + (int64_t)(D2 >> 6);
-  const uint32_t up = (uint32_t)(q >> 63);  // 1: quotient in [1, 2), 0: in (1/2, 1)
-  const uint32_t half = 512u << up;
-  uint64_t m = (q + half) >> (10 + up);
-  if ((((uint32_t)q + half + 3u) & (2u * half - 1u)) < 6u) {
+  const DivDigits d(a, b);
+  if (!d.normal()) return div_rn_slow(a, b);
+  uint64_t m = d.rounded();
+  if (d.close()) {
     // mm - 1/2 is the midpoint next to q
-    const uint64_t mm = (q + half + 3u) >> (10 + up);
-    const int64_t rem = (int64_t)((ma << (54 - up)) - (2 * mm - 1) * mb);
+    const uint64_t mm = (d.q + d.half + 3u) >> (10 + d.up);
+    const int64_t rem = (int64_t)((d.ma << (54 - d.up)) - (2 * mm - 1) * d.mb);
     m = mm - (rem < 0);
   }
-  const uint32_t ex = ea - eb + 1021u + up;
-  const uint32_t hi = ((uint32_t)(m >> 32) + (ex << 20)) | ((ah ^ bh) & 0x80000000u);
-  return __hiloint2double((int)hi, (int)(uint32_t)m);
+  return d.result(m);
+}
+
+// The common case of a / b without a branch, so that several overlap: where
+// `ok` is false (6 in 1000 quotients lie close to a midpoint) the result is to
+// be formed by div_rn.
+__device__ __forceinline__ double div_try(double a, double b, bool& ok) {
+  const DivDigits d(a, b);
+  ok = d.normal() && !d.close();
+  return d.result(d.rounded());
 }
 
 // sqrt(a), the bits of __dsqrt_rn: m = M / 2^52 in [1, 4), root digits S0 at

@@ -158,30 +158,62 @@ __global__ void __launch_bounds__(kBlock)
 // (every cell's factored value is written once, by its own step, and read
 // only by cells after it).  The subtractions of dic_cell, in slot order: a
 // pass first issues the loads of every slot still pending (they are
-// independent, so their round trips overlap), forms the quotient of each that
-// has arrived, then subtracts the quotients in order up to the first one still
-// empty.  The chain from level to level is what bounds the walk, so a*a is
-// formed before the wait and the divisions run on the integer pipe (303 clocks
-// against 560, and several at once).  Cells with more than four
+// independent, so their round trips overlap); when the last has arrived the
+// quotients are formed together and subtracted in order.  The chain from level
+// to level is what bounds the walk, so a*a is formed before the wait and the
+// divisions run on the integer pipe (303 clocks against 560, and several at
+// once).  Cells with more than four
 // neighbour-side slots (polyhedral meshes) walk them one load at a time.
+// The factored value of a cell from the a*a and the v of its first N
+// neighbour-side slots, for the whole warp at once without branches: the
+// quotients overlap (three of them in 400 clocks), and an FP64 instruction
+// that no lane needs would hold the warp all the same.  A lane with nothing to
+// divide divides 1 by 1: an empty slot's NaN or a zero would take the whole
+// warp through the division's slow path.
+template <int N>
+__device__ __forceinline__ double dic_finish(double dc, const double (&a)[4], const double (&v)[4],
+                                             unsigned used, bool finish) {
+  double w[N], p[N], q[N];
+  bool take[N], ok[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    take[k] = finish && (used >> k & 1u) && above_tiny(fabs(v[k]));
+    p[k] = take[k] ? a[k] : 1.0;
+    q[k] = take[k] ? v[k] : 1.0;
+    w[k] = div_try(p[k], q[k], ok[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (!ok[k]) w[k] = div_rn(p[k], q[k]);
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double u = __dsub_rn(dc, w[k]);
+    dc = take[k] ? u : dc;
+  }
+  return dc;
+}
+
+// LOCAL: a block walk (wavefront.cuh), cells in the order of block_ptr
+// (32^3: 229 -> 107 us; 24 systems of 16^3 to 48^3: 385 -> 193 us).
+template <bool LOCAL>
 __global__ void __launch_bounds__(kBlock)
     dic_flow_kernel(gbf_layout L, const double* __restrict__ coef,
                     const double* __restrict__ diag, const int32_t* __restrict__ cells,
-                    double* d, GridBarrier* bar, long long max_polls) {
-  const int n = L.n_cells;
+                    const int32_t* __restrict__ block_ptr, int per, double* d, GridBarrier* bar,
+                    long long max_polls) {
+  extern __shared__ double dyn[];
+  FlowSlots<LOCAL> slots;
+  const FlowRange range = flow_begin<LOCAL>(slots, d, L.n_cells, block_ptr, per, dyn);
   const int lane = threadIdx.x & 31;
-  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long chunks = ((long long)n + 31) >> 5;
   long long polls = 0;
-  for (long long ch = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < chunks;
-       ch += warps) {
-    const long long i = ch * 32 + lane;
-    bool done = i >= n;
+  for (long long at = range.first; at < range.end; at += range.stride) {
+    const long long i = at + lane;
+    bool done = i >= range.end;
     int c = 0, k = 0, wn = 0, base = 0;
     double dc = 0.0;
-    int j[4] = {-1, -1, -1, -1};
-    double a[4] = {0.0, 0.0, 0.0, 0.0};  // a * a, then the quotient
-    unsigned wait = 0, take = 0;         // slots still empty; slots with a quotient
+    double a[4] = {0.0, 0.0, 0.0, 0.0}, v[4] = {1.0, 1.0, 1.0, 1.0};  // a * a; factored values
+    const double* from[4] = {};
+    unsigned used = 0, left = 0;  // slots with a face; with a value still to come
     if (!done) {
       c = __ldg(cells + i);
       dc = __ldg(diag + c);
@@ -191,77 +223,66 @@ __global__ void __launch_bounds__(kBlock)
         base = cs.base + 32 * cs.wo;
       }
       if (wn <= 4) {
-        double dv[4];
+        int j[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          if (q < wn) {
-            j[q] = __ldg(L.slot_col + base + 32 * q);
-            a[q] = __ldg(coef + base + 32 * q);
-          }
+          j[q] = q < wn ? __ldg(L.slot_col + base + 32 * q) : -1;
+          a[q] = q < wn ? __ldg(coef + base + 32 * q) : 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dv[q] = j[q] > c ? __ldg(diag + j[q]) : 0.0;  // unfactored
-#pragma unroll
         for (int q = 0; q < 4; ++q) {
-          if (j[q] < 0) continue;
-          a[q] = __dmul_rn(a[q], a[q]);
-          if (j[q] < c) {
-            wait |= 1u << q;
-          } else if (above_tiny(fabs(dv[q]))) {
-            a[q] = div_rn(a[q], dv[q]);
-            take |= 1u << q;
+          if (j[q] >= 0) used |= 1u << q;
+          if (j[q] > c) v[q] = __ldg(diag + j[q]);  // unfactored
+          if (j[q] >= 0 && j[q] < c) {
+            left |= 1u << q;
+            from[q] = slots.at(j[q]);
           }
+          a[q] = __dmul_rn(a[q], a[q]);
         }
       }
     }
+    const bool few = wn <= 4;
+    const int most = __reduce_max_sync(0xffffffffu, few ? wn : 0);
     bool quit = false;
     for (;;) {
-      if (!done) {
-        if (wn <= 4) {
-          if (wait) {
-            double v[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = (wait >> q & 1u) ? ld_flow(d + j[q]) : 0.0;
+      for (int q = 0; q < 4; ++q)
+        if (left >> q & 1u) v[q] = slots.load(from[q]);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if ((wait >> q & 1u) && !flow_empty(v[q])) {
-                wait &= ~(1u << q);
-                if (above_tiny(fabs(v[q]))) {
-                  a[q] = div_rn(a[q], v[q]);
-                  take |= 1u << q;
-                }
-              }
-          }
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (k == q && q < wn && !(wait >> q & 1u)) {
-              if (take >> q & 1u) dc = __dsub_rn(dc, a[q]);
-              k = q + 1;
-            }
-        } else {
-          for (; k < wn; ++k) {
-            const int s = base + 32 * k;
-            const int jk = __ldg(L.slot_col + s);
-            if (jk < 0) continue;
-            double dj;
-            if (jk < c) {
-              dj = ld_flow(d + jk);
-              if (flow_empty(dj)) break;  // not factored yet: next pass
-            } else {
-              dj = __ldg(diag + jk);
-            }
-            if (above_tiny(fabs(dj))) {
-              const double ak = __ldg(coef + s);
-              dc = __dsub_rn(dc, div_rn(__dmul_rn(ak, ak), dj));
-            }
-          }
-        }
-        if (k >= wn) {
-          st_flow(d + c, dc);
+      for (int q = 0; q < 4; ++q)
+        if ((left >> q & 1u) && !flow_empty(v[q])) left &= ~(1u << q);
+      bool finish = few && !done && left == 0;
+      if (__any_sync(0xffffffffu, finish)) {
+        const double t = most <= 3 ? dic_finish<3>(dc, a, v, used, finish)
+                                   : dic_finish<4>(dc, a, v, used, finish);
+        if (finish) {
+          slots.store(c, t);
           done = true;
         }
       }
-      if (flow_pass_end(done, polls, max_polls, bar, &quit)) break;
+      if (!few && !done) {
+        for (; k < wn; ++k) {
+          const int s = base + 32 * k;
+          const int jk = __ldg(L.slot_col + s);
+          if (jk < 0) continue;
+          double dj;
+          if (jk < c) {
+            dj = slots.load(slots.at(jk));
+            if (flow_empty(dj)) break;  // not factored yet: next pass
+          } else {
+            dj = __ldg(diag + jk);
+          }
+          if (above_tiny(fabs(dj))) {
+            const double ak = __ldg(coef + s);
+            dc = __dsub_rn(dc, div_rn(__dmul_rn(ak, ak), dj));
+          }
+        }
+        if (k >= wn) {
+          slots.store(c, dc);
+          done = true;
+        }
+      }
+      if (flow_pass_end<!LOCAL>(done, polls, max_polls, bar, &quit)) break;
       if (quit) return;
     }
   }
@@ -475,28 +496,56 @@ extern "C" int gbf_dilu_build_f64(const gbf_layout* L, const double* lower, cons
 // runs short at 256^3 (DIC 3.0 ms on 152 blocks, 3.4 on 114, 4.4 on 76).
 static int flow_blocks_per_sm() { return 1; }
 
-extern "C" int gbf_dic_build_flow_f64(const gbf_layout* L, const double* coef, const double* diag,
-                                      const int32_t* level_cells, double* d_out, void* barrier,
-                                      void* stream) {
-  ::gbf::NvtxScope nvtx_("gbf_dic_build_flow_f64");
+// The walk over the whole level schedule (block_ptr NULL), or by blocks.
+static int dic_walk(const char* what, const gbf_layout* L, const double* coef, const double* diag,
+                    const int32_t* cells, const int32_t* block_ptr, int32_t n_blocks, int32_t per,
+                    double* d_out, void* barrier, void* stream) {
   int rc = check_layout(L);
   if (rc) return rc;
   const int n = L->n_cells;
   if (n == 0) return GBF_OK;
-  GBF_REQUIRE(diag && d_out && level_cells && barrier, "dic_build_flow: NULL pointer");
-  GBF_REQUIRE(L->n_faces == 0 || coef, "dic_build_flow: NULL coefficients");
+  GBF_REQUIRE(diag && d_out && cells && barrier, "%s: NULL pointer", what);
+  GBF_REQUIRE(L->n_faces == 0 || coef, "%s: NULL coefficients", what);
   cudaStream_t s = as_stream(stream);
-  const int grid = flow_grid((const void*)dic_flow_kernel, n, flow_blocks_per_sm());
-  GBF_REQUIRE(grid > 0, "dic_build_flow: the device cannot launch cooperative kernels");
   GBF_CHECK_CUDA(cudaMemsetAsync(d_out, 0xff, sizeof(double) * (size_t)n, s));
   gbf_layout Lc = *L;
   GridBarrier* bar = static_cast<GridBarrier*>(barrier);
   long long polls = kFlowPolls;
-  void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&level_cells, &d_out, &bar, &polls};
-  GBF_CHECK_CUDA(launch_wavefront((const void*)dic_flow_kernel, grid, args, barrier, s));
+  void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&cells, (void*)&block_ptr,
+                  &per, &d_out, &bar, &polls};
+  if (block_ptr) {
+    GBF_CHECK_CUDA(launch_walk((const void*)dic_flow_kernel<true>, n_blocks, per, args, barrier, s));
+  } else {
+    const int grid = flow_grid((const void*)dic_flow_kernel<false>, n, flow_blocks_per_sm());
+    GBF_REQUIRE(grid > 0, "%s: the device cannot launch cooperative kernels", what);
+    GBF_CHECK_CUDA(launch_wavefront((const void*)dic_flow_kernel<false>, grid, args, barrier, s));
+  }
   dic_flow_out_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(n, bar, d_out);
   GBF_CHECK_LAUNCH();
   return GBF_OK;
+}
+
+extern "C" int gbf_dic_build_flow_f64(const gbf_layout* L, const double* coef, const double* diag,
+                                      const int32_t* level_cells, double* d_out, void* barrier,
+                                      void* stream) {
+  ::gbf::NvtxScope nvtx_("gbf_dic_build_flow_f64");
+  return dic_walk("dic_build_flow", L, coef, diag, level_cells, nullptr, 0, 0, d_out, barrier,
+                  stream);
+}
+
+extern "C" int gbf_dic_build_block_f64(const gbf_layout* L, const double* coef, const double* diag,
+                                       const int32_t* block_cells, const int32_t* block_ptr,
+                                       int32_t n_blocks, int32_t per, double* d_out, void* barrier,
+                                       void* stream) {
+  ::gbf::NvtxScope nvtx_("gbf_dic_build_block_f64");
+  GBF_REQUIRE(L && block_ptr, "dic_build_block: NULL pointer");
+  GBF_REQUIRE(n_blocks >= 1 && per >= 1 && per <= kWalkCellsMax &&
+                  (long long)n_blocks * per >= L->n_cells &&
+                  (long long)(n_blocks - 1) * per < (L->n_cells > 0 ? L->n_cells : 1),
+              "dic_build_block: %d blocks of %d cells do not cover %d cells", n_blocks, per,
+              L->n_cells);
+  return dic_walk("dic_build_block", L, coef, diag, block_cells, block_ptr, n_blocks, per, d_out,
+                  barrier, stream);
 }
 
 extern "C" size_t gbf_dilu_flow_slots_bytes(int32_t n_faces) {

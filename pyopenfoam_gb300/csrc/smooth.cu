@@ -153,116 +153,163 @@ __global__ void __launch_bounds__(kBlock)
 // What bounds it is the chain from one level to the next: the store, its
 // neighbour's poll, and the FP64 operations between them, 64 clocks each (a
 // CUDA divide 560).  So everything that does not need a new value happens
-// before the wait -- loads, the products with old values, the sum up to the
-// first new value -- a pass only polls what is still missing, and an arrival
-// costs its product, the rest of the row's additions and one integer-pipe
-// division.  Repeating gs_row on every pass instead took 5.1 us a level
-// (67 x 59 x 53 cells: 902 us a sweep, 466 us now).  The products, their order
+// before the wait -- loads, the products with old values -- a pass only polls
+// what is still missing, and the last arrival is followed by the products with
+// new values, the row's additions and one integer-pipe division.  Repeating
+// gs_row on every pass instead took 5.1 us a level
+// (67 x 59 x 53 cells: 902 us a sweep, 274 us now).  The products, their order
 // and the update are gs_cell's (gs_row, gs_update): the same bits.  Cells with
 // more than four slots a side, and cells whose owner-side faces do not all
 // follow their neighbour-side faces, repeat gs_row.
-template <bool RELAX>
+//
+// The row sum of a cell from its first N slots a side, for the whole warp at
+// once without branches (an FP64 instruction that no lane needs would hold the
+// warp all the same): the waited-for side's products, then the terms in order.
+template <int N>
+__device__ __forceinline__ double gs_finish(double row, const double (&pn)[4],
+                                            const double (&po)[4], const double (&v)[4],
+                                            unsigned used, unsigned wait, bool reverse) {
+  double t[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double c = reverse ? po[k] : pn[k], p = __dmul_rn(c, v[k]);
+    t[k] = (wait >> k & 1u) ? p : c;
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double s = __dadd_rn(row, reverse ? pn[k] : t[k]);
+    row = (used >> k & 1u) ? s : row;
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    const double s = __dadd_rn(row, reverse ? t[k] : po[k]);
+    row = (used >> k & 16u) ? s : row;
+  }
+  return row;
+}
+
+// LOCAL: a block walk (wavefront.cuh), cells in the order of block_ptr.
+template <bool RELAX, bool LOCAL>
 __global__ void __launch_bounds__(kBlock)
     gs_flow_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
-                   const double* __restrict__ b, const int32_t* __restrict__ cells, int reverse,
-                   double omega, const double* __restrict__ x_old, double* x_new,
-                   GridBarrier* bar, long long max_polls) {
-  const int n = L.n_cells;
+                   const double* __restrict__ b, const int32_t* __restrict__ cells,
+                   const int32_t* __restrict__ block_ptr, int per, int reverse, double omega,
+                   const double* __restrict__ x_old, double* x_new, GridBarrier* bar,
+                   long long max_polls) {
+  extern __shared__ double dyn[];
+  FlowSlots<LOCAL> slots;
+  const FlowRange range = flow_begin<LOCAL>(slots, x_new, L.n_cells, block_ptr, per, dyn);
   const int lane = threadIdx.x & 31;
-  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long chunks = ((long long)n + 31) >> 5;
   long long polls = 0;
-  for (long long ch = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < chunks;
-       ch += warps) {
-    const long long i = ch * 32 + lane;
-    bool done = i >= n;
+  for (long long at = range.first; at < range.end; at += range.stride) {
+    const long long i = at + lane;
+    bool done = i >= range.end;
     int c = 0;
     double dc = 0.0, xc = 0.0, bc = 0.0;
-    // slots in face order: position o is neighbour-side slot o (o < 4), then
-    // owner-side slot o - 4
+    // pn, po: coefficients of the neighbour- and owner-side slots, of old
+    // values already times the value; `from` where a new value is polled
     bool ordered = false;
-    unsigned used = 0, wait = 0;  // positions with a face; with a new value still to come
-    int q[8];
-    double p[8], row = 0.0, dx = 0.0;  // p: the product, or the coefficient while waiting
-    int pos = 0;
+    unsigned used = 0, wait = 0;  // bit k: neighbour-side slot k, 4 + k: owner-side slot k
+    double pn[4] = {}, po[4] = {}, v[4] = {}, dx = 0.0;
+    const double* from[4] = {};
+    int wo = 0, wn = 0;
     if (!done) {
       c = __ldg(cells + i);
       dc = __ldg(diag + c);
       xc = __ldg(x_old + c);
       bc = __ldg(b + c);
+      ordered = L.n_faces == 0;
       if (L.n_faces > 0) {
         const CellSlots cs = cell_slots(L, c);
         if (cs.wo <= 4 && cs.wn <= 4) {
-          int max_nei = -1, min_own = INT_MAX;
+          wo = cs.wo;
+          wn = cs.wn;
+          int fn[4], fo[4], qn[4], qo[4];
 #pragma unroll
-          for (int o = 0; o < 8; ++o) {
-            const bool use = o < 4 ? o < cs.wn : o - 4 < cs.wo;
-            const int k = o < 4 ? cs.wo + o : o - 4;
-            const int slot = cs.base + 32 * k;
-            const int f = use ? __ldg(L.slot_face + slot) : -1;
-            q[o] = use ? slot_column(L, cs.e0 + k, slot, c) : -1;
-            p[o] = use ? __ldg(coef + slot) : 0.0;
-            if (f >= 0 && q[o] >= 0) {
-              used |= 1u << o;
-              if (reverse ? q[o] > c : q[o] < c) wait |= 1u << o;
-              if (o < 4) max_nei = f;
-              else if (min_own == INT_MAX) min_own = f;
-            }
+          for (int k = 0; k < 4; ++k) {
+            const int so = cs.base + 32 * k, sn = cs.base + 32 * (wo + k);
+            fo[k] = k < wo ? __ldg(L.slot_face + so) : -1;
+            fn[k] = k < wn ? __ldg(L.slot_face + sn) : -1;
+            qo[k] = k < wo ? slot_column(L, cs.e0 + k, so, c) : -1;
+            qn[k] = k < wn ? slot_column(L, cs.e0 + wo + k, sn, c) : -1;
+            po[k] = k < wo ? __ldg(coef + so) : 0.0;
+            pn[k] = k < wn ? __ldg(coef + sn) : 0.0;
           }
-          ordered = max_nei < min_own;
+          // forward sweeps wait on the neighbour side, backward on the owner side
+          bool usual = true;
+          int max_nei = -1, min_own = INT_MAX;
+          double xo[4], xn[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const bool un = fn[k] >= 0 && qn[k] >= 0, uo = fo[k] >= 0 && qo[k] >= 0;
+            if (un) used |= 1u << k, max_nei = fn[k];
+            if (uo) used |= 16u << k, min_own = min_own < fo[k] ? min_own : fo[k];
+            const bool nn = un && (reverse ? qn[k] > c : qn[k] < c);
+            const bool no = uo && (reverse ? qo[k] > c : qo[k] < c);
+            if (reverse ? nn : no) usual = false;
+            if (reverse ? no : nn) {
+              wait |= 1u << k;
+              from[k] = slots.at(reverse ? qo[k] : qn[k]);
+            }
+            xn[k] = un && !nn ? __ldg(x_old + qn[k]) : 1.0;
+            xo[k] = uo && !no ? __ldg(x_old + qo[k]) : 1.0;
+          }
+          ordered = usual && max_nei < min_own;
           if (ordered) {
-            double v[8];
 #pragma unroll
-            for (int o = 0; o < 8; ++o)
-              v[o] = ((used & ~wait) >> o & 1u) ? __ldg(x_old + q[o]) : 0.0;
-#pragma unroll
-            for (int o = 0; o < 8; ++o)
-              if ((used & ~wait) >> o & 1u) p[o] = __dmul_rn(p[o], v[o]);
+            for (int k = 0; k < 4; ++k) {
+              if (reverse || !(wait >> k & 1u)) pn[k] = __dmul_rn(pn[k], xn[k]);
+              if (!reverse || !(wait >> k & 1u)) po[k] = __dmul_rn(po[k], xo[k]);
+            }
+          } else {
+            wait = 0;
           }
         }
       }
       dx = __dmul_rn(dc, xc);
-      row = dx;
     }
+    unsigned left = wait;
+    const int most_n = __reduce_max_sync(0xffffffffu, wn);
+    const int most_o = __reduce_max_sync(0xffffffffu, wo);
     bool quit = false;
     for (;;) {
-      if (!done) {
-        bool missing = false;
-        if (ordered) {
-          if (wait) {
-            double v[8];
 #pragma unroll
-            for (int o = 0; o < 8; ++o) v[o] = (wait >> o & 1u) ? ld_flow(x_new + q[o]) : 0.0;
+      for (int k = 0; k < 4; ++k)
+        if (left >> k & 1u) v[k] = slots.load(from[k]);
 #pragma unroll
-            for (int o = 0; o < 8; ++o)
-              if ((wait >> o & 1u) && !flow_empty(v[o])) {
-                p[o] = __dmul_rn(p[o], v[o]);
-                wait &= ~(1u << o);
-              }
-          }
-#pragma unroll
-          for (int o = 0; o < 8; ++o)
-            if (pos == o && !(wait >> o & 1u)) {
-              if (used >> o & 1u) row = __dadd_rn(row, p[o]);
-              pos = o + 1;
-            }
-          missing = pos < 8;
-        } else {
-          row = gs_row(L, coef, dc, xc, c, [&](int col) {
-            if (reverse ? col > c : col < c) {
-              const double v = ld_flow(x_new + col);
-              missing |= flow_empty(v);
-              return v;
-            }
-            return __ldg(x_old + col);
-          });
-        }
-        if (!missing) {
-          st_flow(x_new + c, gs_update<RELAX>(row, dx, dc, xc, bc, omega));
+      for (int k = 0; k < 4; ++k)
+        if ((left >> k & 1u) && !flow_empty(v[k])) left &= ~(1u << k);
+      bool finish = ordered && !done && left == 0;
+      if (__any_sync(0xffffffffu, finish)) {
+        const double row =
+            most_n <= 3 && most_o <= 3
+                ? gs_finish<3>(dx, pn, po, v, used, wait, reverse)
+                : gs_finish<4>(dx, pn, po, v, used, wait, reverse);
+        // a lane that does not finish divides 1 by 1: an empty slot's NaN would
+        // take the whole warp through the division's slow path
+        const double nv = gs_update<RELAX>(finish ? row : dx, dx, finish ? dc : 1.0, xc,
+                                           finish ? bc : 1.0, omega);
+        if (finish) {
+          slots.store(c, nv);
           done = true;
         }
       }
-      if (flow_pass_end(done, polls, max_polls, bar, &quit)) break;
+      if (!ordered && !done) {
+        bool missing = false;
+        const double row = gs_row(L, coef, dc, xc, c, [&](int col) {
+          if (reverse ? col > c : col < c) {
+            const double w = slots.load(slots.at(col));
+            missing |= flow_empty(w);
+            return w;
+          }
+          return __ldg(x_old + col);
+        });
+        if (!missing) {
+          slots.store(c, gs_update<RELAX>(row, dx, dc, xc, bc, omega));
+          done = true;
+        }
+      }
+      if (flow_pass_end<!LOCAL>(done, polls, max_polls, bar, &quit)) break;
       if (quit) return;
     }
   }
@@ -552,36 +599,70 @@ extern "C" int gbf_gauss_seidel_f64(const gbf_layout* L, const double* coef, con
   return GBF_OK;
 }
 
-extern "C" int gbf_gauss_seidel_flow_f64(const gbf_layout* L, const double* coef,
-                                         const double* diag, const double* b,
-                                         const int32_t* level_cells, int32_t reverse,
-                                         double omega, int32_t relax, double* x, double* scratch,
-                                         void* barrier, void* stream) {
-  ::gbf::NvtxScope nvtx_("gbf_gauss_seidel_flow_f64");
+// The walk over the whole level schedule (block_ptr NULL), or by blocks.
+static int gauss_seidel_walk(const char* what, const gbf_layout* L, const double* coef,
+                             const double* diag, const double* b, const int32_t* cells,
+                             const int32_t* block_ptr, int32_t n_blocks, int32_t per,
+                             int32_t reverse, double omega, int32_t relax, double* x,
+                             double* scratch, void* barrier, void* stream) {
   int rc = check_layout(L);
   if (rc) return rc;
   const int n = L->n_cells;
   if (n == 0) return GBF_OK;
-  GBF_REQUIRE(diag && b && x && level_cells && scratch && barrier && (L->n_faces == 0 || coef),
-              "gauss_seidel_flow: NULL pointer");
-  GBF_REQUIRE(scratch != x, "gauss_seidel_flow: scratch must not be x");
+  GBF_REQUIRE(diag && b && x && cells && scratch && barrier && (L->n_faces == 0 || coef),
+              "%s: NULL pointer", what);
+  GBF_REQUIRE(scratch != x, "%s: scratch must not be x", what);
   cudaStream_t s = as_stream(stream);
-  const void* k = relax ? (const void*)gs_flow_kernel<true> : (const void*)gs_flow_kernel<false>;
-  // one block per SM (the polling of warps ahead of the front slows it)
-  const int grid = wavefront_grid(k, kBlock, n, 1);
-  GBF_REQUIRE(grid > 0, "gauss_seidel_flow: the device cannot launch cooperative kernels");
   GBF_CHECK_CUDA(cudaMemsetAsync(scratch, 0xff, sizeof(double) * (size_t)n, s));
   gbf_layout Lc = *L;
   int rev = reverse != 0;
   long long polls = kFlowPolls;
   GridBarrier* bar = static_cast<GridBarrier*>(barrier);
   const double* xo = x;
-  void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&b, (void*)&level_cells, &rev,
-                  &omega, (void*)&xo, &scratch, &bar, &polls};
-  GBF_CHECK_CUDA(launch_wavefront(k, grid, args, barrier, s));
+  void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&b, (void*)&cells, (void*)&block_ptr,
+                  &per, &rev, &omega, (void*)&xo, &scratch, &bar, &polls};
+  if (block_ptr) {
+    const void* k = relax ? (const void*)gs_flow_kernel<true, true>
+                          : (const void*)gs_flow_kernel<false, true>;
+    GBF_CHECK_CUDA(launch_walk(k, n_blocks, per, args, barrier, s));
+  } else {
+    const void* k = relax ? (const void*)gs_flow_kernel<true, false>
+                          : (const void*)gs_flow_kernel<false, false>;
+    // one block per SM (the polling of warps ahead of the front slows it)
+    const int grid = wavefront_grid(k, kBlock, n, 1);
+    GBF_REQUIRE(grid > 0, "%s: the device cannot launch cooperative kernels", what);
+    GBF_CHECK_CUDA(launch_wavefront(k, grid, args, barrier, s));
+  }
   gs_flow_out_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(n, bar, scratch, x);
   GBF_CHECK_LAUNCH();
   return GBF_OK;
+}
+
+extern "C" int gbf_gauss_seidel_flow_f64(const gbf_layout* L, const double* coef,
+                                         const double* diag, const double* b,
+                                         const int32_t* level_cells, int32_t reverse,
+                                         double omega, int32_t relax, double* x, double* scratch,
+                                         void* barrier, void* stream) {
+  ::gbf::NvtxScope nvtx_("gbf_gauss_seidel_flow_f64");
+  return gauss_seidel_walk("gauss_seidel_flow", L, coef, diag, b, level_cells, nullptr, 0, 0,
+                           reverse, omega, relax, x, scratch, barrier, stream);
+}
+
+extern "C" int gbf_gauss_seidel_block_f64(const gbf_layout* L, const double* coef,
+                                          const double* diag, const double* b,
+                                          const int32_t* block_cells, const int32_t* block_ptr,
+                                          int32_t n_blocks, int32_t per, int32_t reverse,
+                                          double omega, int32_t relax, double* x, double* scratch,
+                                          void* barrier, void* stream) {
+  ::gbf::NvtxScope nvtx_("gbf_gauss_seidel_block_f64");
+  GBF_REQUIRE(L && block_ptr, "gauss_seidel_block: NULL pointer");
+  GBF_REQUIRE(n_blocks >= 1 && per >= 1 && per <= kWalkCellsMax &&
+                  (long long)n_blocks * per >= L->n_cells &&
+                  (long long)(n_blocks - 1) * per < (L->n_cells > 0 ? L->n_cells : 1),
+              "gauss_seidel_block: %d blocks of %d cells do not cover %d cells", n_blocks, per,
+              L->n_cells);
+  return gauss_seidel_walk("gauss_seidel_block", L, coef, diag, b, block_cells, block_ptr,
+                           n_blocks, per, reverse, omega, relax, x, scratch, barrier, stream);
 }
 
 extern "C" int gbf_residual_f64(const gbf_layout* L, const double* coef, const double* diag,

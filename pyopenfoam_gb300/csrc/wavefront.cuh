@@ -92,8 +92,15 @@ __device__ __forceinline__ double ld_flow(const double* p) {
   return v;
 }
 
+// v, a NaN as the canonical one (compared as integers: an FP64 instruction,
+// a compare too, holds the warp for 64 clocks on GB300).
+__device__ __forceinline__ double flow_value(double v) {
+  const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+  return b > 0x7ff0000000000000LL ? __longlong_as_double(0x7ff8000000000000LL) : v;
+}
+
 __device__ __forceinline__ void st_flow(double* p, double v) {
-  if (v != v) v = __longlong_as_double(0x7ff8000000000000LL);
+  v = flow_value(v);
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
@@ -101,8 +108,84 @@ __device__ __forceinline__ bool flow_empty(double v) {
   return __double_as_longlong(v) == kFlowEmpty;
 }
 
+// ---- block walks -------------------------------------------------------------
+//
+// A dataflow walk whose block b takes the cells [b per, (b+1) per) and keeps
+// their slots in shared memory as well: a step whose inputs come from cells of
+// its own block polls those (30 clocks) instead of a store's and a load's trip
+// through L2 (together some 1500).  With cells numbered so that neighbours are
+// mostly close -- any mesh numbering used in earnest -- most links of the chain
+// from level to level stay inside a block.  Each block's items are in level
+// order, 32 at a time round-robin to its warps; the warp holding the globally
+// earliest unfinished item finds its inputs, as in the walk over the whole
+// schedule: its block has begun every chunk before that one, and they are done.
+constexpr int kWalkCellsMax = 24576;  // cells per block: 192 KB of slots
+
+// The slots of one walk, as one block sees them.
+template <bool LOCAL>
+struct FlowSlots {
+  double* g;       // all slots, in device memory
+  double* own;     // this block's, in shared memory
+  int c0, count;   // its cells
+
+  // Where c's value is polled: a generic address, so that a warp's polls of
+  // both kinds are one load instruction without a branch.
+  __device__ __forceinline__ const double* at(int c) const {
+    return LOCAL && (unsigned)(c - c0) < (unsigned)count ? own + (c - c0) : g + c;
+  }
+  static __device__ __forceinline__ double load(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    return v;
+  }
+  // c is one of this block's cells when LOCAL
+  __device__ __forceinline__ void store(int c, double v) const {
+    v = flow_value(v);
+    if (LOCAL) asm volatile("st.relaxed.gpu.f64 [%0], %1;" ::"l"(own + (c - c0)), "d"(v) : "memory");
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(g + c), "d"(v) : "memory");
+  }
+};
+
+// The items a warp takes: 32 at `first`, `stride` further on, up to `end`.
+struct FlowRange {
+  long long first, end, stride;
+};
+
+// Sets up a walk over `n` items (LOCAL: those of item_ptr[block] on, cells of
+// `per` a block, with `dyn` the block's shared memory).
+template <bool LOCAL>
+__device__ __forceinline__ FlowRange flow_begin(FlowSlots<LOCAL>& slots, double* g, int n,
+                                                const int32_t* __restrict__ item_ptr, int per,
+                                                double* dyn) {
+  slots.g = g;
+  const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  if (!LOCAL)
+    return FlowRange{32LL * (blockIdx.x * warps + warp), n, 32LL * gridDim.x * warps};
+  slots.c0 = blockIdx.x * per;
+  slots.count = n - slots.c0 < per ? n - slots.c0 : per;
+  slots.own = dyn;
+  for (int i = threadIdx.x; i < slots.count; i += blockDim.x)
+    dyn[i] = __longlong_as_double(kFlowEmpty);
+  __syncthreads();
+  const long long b = __ldg(item_ptr + blockIdx.x);
+  return FlowRange{b + 32 * warp, __ldg(item_ptr + blockIdx.x + 1), 32LL * warps};
+}
+
+// Launches a block walk: `n_blocks` resident blocks with `per` slots each.
+inline cudaError_t launch_walk(const void* kernel, int n_blocks, int per, void** args,
+                               void* barrier, cudaStream_t s) {
+  const size_t dyn = sizeof(double) * (size_t)per;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(sizeof(double) * kWalkCellsMax));
+  if (e == cudaSuccess) e = cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), s);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchCooperativeKernel(kernel, dim3(n_blocks), dim3(kBlock), args, dyn, s);
+}
+
 // End of one pass over a chunk: true when every lane is done; false with
-// *quit set when a wait ran out here or elsewhere.
+// *quit set when a wait ran out here or elsewhere.  SLEEP: whether the pass
+// pauses (a walk that polls shared memory does not).
+template <bool SLEEP = true>
 __device__ __forceinline__ bool flow_pass_end(bool done, long long& polls, long long max_polls,
                                               GridBarrier* bar, bool* quit) {
   if (__all_sync(0xffffffffu, done)) return true;
@@ -119,7 +202,7 @@ __device__ __forceinline__ bool flow_pass_end(bool done, long long& polls, long 
   }
   // the pass is bound by the polls' L2 round trip: 0, 16 or 64 ns of sleep
   // measured the same on GB300 (DILU 128^3 2.61-2.62 ms), 256 ns 2 % slower
-  __nanosleep(64);
+  if (SLEEP) __nanosleep(64);
   return false;
 }
 

@@ -55,7 +55,13 @@ def factor_dic(topo, coef: torch.Tensor, diag: torch.Tensor, d: torch.Tensor, de
     sched = topo.dic_schedule()
     L, st = _lib.lib(), _lib.stream_ptr(device)
     bar = None if form == "per_level" else _lib.wavefront_barrier(device)
-    if form == "flow":
+    blocks = topo.dic_blocks() if form == "flow" else None
+    if blocks is not None:
+        _lib.check(L.gbf_dic_build_block_f64(topo.layout_ref, coef.data_ptr(), diag.data_ptr(),
+                                             blocks.cells.data_ptr(), blocks.ptr.data_ptr(),
+                                             blocks.n_blocks, blocks.per, d.data_ptr(),
+                                             bar.data_ptr(), st), "gbf_dic_build_block_f64")
+    elif form == "flow":
         _lib.check(L.gbf_dic_build_flow_f64(topo.layout_ref, coef.data_ptr(), diag.data_ptr(),
                                             sched.items.data_ptr(), d.data_ptr(),
                                             bar.data_ptr(), st), "gbf_dic_build_flow_f64")

@@ -22,6 +22,7 @@ import torch
 
 from .. import _lib
 from ..core.ldu_matrix import LduMatrix
+from ..core.topology import block_order
 from .preconditioners import DICPreconditioner
 
 __all__ = ["Smoother", "GaussSeidelSmoother", "JacobiSmoother", "DICGSmoother", "gs_sweep",
@@ -58,6 +59,7 @@ class _GsSchedule:
         self.ptr_h = np.ascontiguousarray(ptr[: nl.value + 1])
         self.ptr = torch.from_numpy(self.ptr_h.copy()).to(topo.device)
         self.cells = torch.from_numpy(cells).to(topo.device)
+        self.blocks = block_order(cells[:n], topo.device)
 
 
 def _gs_schedule(matrix: LduMatrix, reverse: bool) -> _GsSchedule:
@@ -89,6 +91,15 @@ def gs_sweep(matrix: LduMatrix, x: torch.Tensor, b: torch.Tensor, reverse: bool 
     st = _lib.stream_ptr(matrix.device)
     if form == "flow":
         scratch = torch.empty(max(matrix.n_cells, 1), dtype=torch.float64, device=matrix.device)
+        if sch.blocks is not None:
+            bl = sch.blocks
+            _lib.check(_lib.lib().gbf_gauss_seidel_block_f64(
+                topo.layout_ref, coef.data_ptr(), matrix.diag.data_ptr(), b.data_ptr(),
+                bl.cells.data_ptr(), bl.ptr.data_ptr(), bl.n_blocks, bl.per, int(reverse),
+                float(omega), int(relax), x.data_ptr(), scratch.data_ptr(),
+                _lib.wavefront_barrier(matrix.device).data_ptr(), st),
+                "gbf_gauss_seidel_block_f64")
+            return
         _lib.check(_lib.lib().gbf_gauss_seidel_flow_f64(
             topo.layout_ref, coef.data_ptr(), matrix.diag.data_ptr(), b.data_ptr(),
             sch.cells.data_ptr(), int(reverse), float(omega), int(relax), x.data_ptr(),
