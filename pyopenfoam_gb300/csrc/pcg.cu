@@ -23,6 +23,8 @@
 
 #include "amul.cuh"
 #include "barrier.cuh"
+#include "exact.cuh"
+#include "wavefront.cuh"
 
 namespace gbf {
 
@@ -57,7 +59,7 @@ __global__ void __launch_bounds__(kBlock)
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += G * blockDim.x) {
     const double y = cell_amul<double, double, false>(L, coef, diag, x, c, __ldg(x + c));
     const double rc = __dsub_rn(__ldg(b + c), y);
-    const double zc = PREC ? __ddiv_rn(rc, __ldg(pd + c)) : rc;
+    const double zc = PREC ? div_rn(rc, __ldg(pd + c)) : rc;
     v.r[c] = rc;
     v.z[c] = zc;
     v.p[c] = zc;
@@ -132,7 +134,7 @@ __global__ void __launch_bounds__(kBlock)
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += G * blockDim.x) {
     const double xc = __dadd_rn(x[c], __dmul_rn(alpha, v.p[c]));
     const double rc = __dsub_rn(v.r[c], __dmul_rn(alpha, v.Ap[c]));
-    const double zc = PREC ? __ddiv_rn(rc, __ldg(pd + c)) : rc;
+    const double zc = PREC ? div_rn(rc, __ldg(pd + c)) : rc;
     x[c] = xc;
     v.r[c] = rc;
     v.z[c] = zc;
@@ -190,8 +192,13 @@ __global__ void __launch_bounds__(kBlock) pcg_p_kernel(int n, PcgVecs v) {
 // sees the fault returns within 16 polls.  The host turns a fault into
 // GBF_DEVICE_TIMEOUT.
 // ---------------------------------------------------------------------------
+// Its blocks per SM: the grid decides which cells share a partial sum, so it is
+// fixed here and does not follow the register count of the day.
 template <int KIND, bool PREC>
-__global__ void __launch_bounds__(kBlock)
+constexpr int kPersistentPerSM = !PREC ? 4 : KIND == kLayoutHex33 ? 2 : 3;
+
+template <int KIND, bool PREC>
+__global__ void __launch_bounds__(kBlock, (kPersistentPerSM<KIND, PREC>))
     pcg_persistent_kernel(gbf_layout L, const double* __restrict__ coef,
                           const double* __restrict__ diag, const double* __restrict__ pd,
                           const double* __restrict__ b, double* __restrict__ x, PcgVecs v,
@@ -210,7 +217,7 @@ __global__ void __launch_bounds__(kBlock)
   for (int c = c0; c < n; c += cs) {
     const double y = cell_amul_k<KIND, double, double, false>(L, coef, diag, x, c, __ldg(x + c));
     const double rc = __dsub_rn(__ldg(b + c), y);
-    const double zc = PREC ? __ddiv_rn(rc, __ldg(pd + c)) : rc;
+    const double zc = PREC ? div_rn(rc, __ldg(pd + c)) : rc;
     v.r[c] = rc;
     v.z[c] = zc;
     v.p[c] = zc;
@@ -266,7 +273,7 @@ __global__ void __launch_bounds__(kBlock)
     for (int c = c0; c < n; c += cs) {
       const double xc = __dadd_rn(x[c], __dmul_rn(alpha, __ldcg(v.p + c)));
       const double rc = __dsub_rn(v.r[c], __dmul_rn(alpha, v.Ap[c]));
-      const double zc = PREC ? __ddiv_rn(rc, __ldg(pd + c)) : rc;
+      const double zc = PREC ? div_rn(rc, __ldg(pd + c)) : rc;
       x[c] = xc;
       v.r[c] = rc;
       v.z[c] = zc;
@@ -316,6 +323,377 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same solve for systems whose cells fit one per resident thread (hex 3+3
+// layouts).  At 32^3 an iteration of pcg_persistent_kernel took 15.3 us, of
+// which three grid barriers with a read of the partial sums behind each took
+// about 6 and FP64 instructions -- 64 clocks each on the warp's SM quarter, two
+// warps a quarter -- most of the rest.  Here:
+//   * a thread keeps its cell's coefficients, x, r, z, p and its neighbours' p
+//     in registers; p of the block's own cells is shared, p of the others'
+//     is recomputed from their z (the same two roundings), so that an
+//     iteration exchanges z and the partial sums only and needs two
+//     grid-wide waits instead of three;
+//   * a wait is the exchange of the values itself: z and the blocks' partial
+//     sums travel as 16-byte words of a value and the number of its turn,
+//     written and read whole, and whoever needs a value polls its word until
+//     the turn is right (no counter, no second trip for the values, no fence
+//     on the way, nothing to clear); a block's sums go into a copy for each
+//     block, so no two blocks poll the same lines;
+//   * two sums go through one tree (the halves of a warp), quotients run on
+//     the integer pipe, convergence is one comparison of r.r with the smallest
+//     r.r that is not converged, and x is updated while the sums travel.
+// The partial sums are those of pcg_persistent_kernel, block by block and in
+// its order, so x, the residuals and the decisions are its bits.  An iteration
+// takes 8.6 us at 32^3 (15.3 before) and 14.2 us at 48 x 40 x 36 (23.3); of
+// that some 3.3 and 6.4 us are FP64 instructions.  Tried on the way: sums
+// behind a grid barrier's release and acquire, 11.3 and 20.5 us (a release
+// store waits 2-5 us behind the other blocks' polls); empty-marker slots with
+// a fence per iteration, 9.4 and 17.7 us; every block polling the same words
+// instead of its own copy, 9.3 and 15.2 us.
+//
+// A word is written again two turns later.  Sums: a block publishes its sums of
+// wait w + 2 after it has collected those of w + 1 of every block, and a block
+// publishes those after it has read all of w.  z: a thread publishes that of
+// iteration i + 2 after its block has collected p.Ap of that iteration, and a
+// block publishes its part of it after its threads have read all z of i + 1.
+// ---------------------------------------------------------------------------
+constexpr int kSlotSets = 2;
+
+// A value and the number of its turn.
+struct __align__(16) TurnWord {
+  double v;
+  long long turn;
+};
+
+__device__ __forceinline__ void st_word(TurnWord* p, double v, long long turn) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"(turn)
+      : "memory");
+}
+
+__device__ __forceinline__ TurnWord ld_word(const TurnWord* p) {
+  long long v, turn;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\t"
+      "mov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(v), "=l"(turn)
+      : "l"(p)
+      : "memory");
+  return TurnWord{__longlong_as_double(v), turn};
+}
+
+// Resident blocks per SM the kernel is compiled for: it takes systems of up to
+// 2 * 256 cells per SM (77824 on 152), for which pcg_persistent_kernel, with at
+// least as many blocks resident, has a cell a thread too.
+constexpr int kResidentPerSM = 2;
+constexpr int kResidentMaxBlocks = 512;  // sizes the workspace
+
+// The sums over the block of a and b, each the tree of block_sum: lanes 0-15 of
+// a warp carry a, lanes 16-31 b, so each level is one addition for both.
+// Threads from `count` on hold 0.0.  Valid in threads 0 (a) and 16 (b).
+__device__ __forceinline__ double block_sum_pair(double a, double b, double* sh, int count) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool low = lane < 16;
+  double v = 0.0;
+  if (32 * wid < count) {
+    v = __dadd_rn(low ? a : b, __shfl_xor_sync(0xffffffffu, low ? b : a, 16));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o, 16));
+  }
+  if ((lane & 15) == 0) sh[(low ? 0 : 8) + wid] = v;
+  __syncthreads();
+  if (wid == 0) {
+    // the tree's first two levels add zeros, which turn -0.0 into +0.0
+    v = first_term((lane & 15) < 8 ? sh[(low ? 0 : 8) + (lane & 7)] : 0.0);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o, 16));
+  }
+  return v;
+}
+
+// As above for one sum; valid in thread 0.
+__device__ __forceinline__ double block_sum_one(double v, double* sh, int count) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (32 * wid < count) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+  }
+  if (lane == 0) sh[wid] = v;
+  __syncthreads();
+  if (wid == 0) {
+    v = first_term(lane < 8 ? sh[lane] : 0.0);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = __dadd_rn(v, __shfl_down_sync(0xffffffffu, v, o));
+  }
+  return v;
+}
+
+// One unsuccessful round of polls; false when the wait has run out.
+__device__ __forceinline__ bool poll_again(long long& polls, int* fault) {
+  ++polls;
+  if (polls > kBarrierPolls || ((polls & 63) == 0 && *(volatile int*)fault != 0)) {
+    atomicExch(fault, 1);
+    return false;
+  }
+  return true;
+}
+
+// a < b for a > 0, +0.0 or NaN and b >= +0.0 or NaN, on the integer pipe.
+__device__ __forceinline__ bool less_nn(double a, double b) {
+  const unsigned long long ua = (unsigned long long)__double_as_longlong(a);
+  const unsigned long long ub = (unsigned long long)__double_as_longlong(b);
+  return ua < ub && ub <= 0x7ff0000000000000ull;
+}
+
+// The smallest s >= 0 for which a monotone test holds, from a guess a few
+// representable numbers away at most; NaN when it is not found there.
+template <typename F>
+__device__ __forceinline__ double first_where(double guess, F&& test) {
+  long long g = __double_as_longlong(guess);
+  for (int k = 0; k < 16 && !test(__longlong_as_double(g)); ++k) ++g;
+  for (int k = 0; k < 32; ++k) {
+    if (!test(__longlong_as_double(g))) return __longlong_as_double(0x7ff8000000000000LL);
+    if (g == 0 || !test(__longlong_as_double(g - 1))) return __longlong_as_double(g);
+    --g;
+  }
+  return __longlong_as_double(0x7ff8000000000000LL);
+}
+
+// The smallest r.r whose norm does not satisfy monitor_converged's two norm
+// rules (sqrt and the division by res0 are monotone): 0 when none does, NaN
+// when it lies outside the ordinary range, where the rules are applied as
+// they stand.
+__device__ double unconverged_rr(double res0, const gbf_solve_params& P) {
+  const double nan = __longlong_as_double(0x7ff8000000000000LL);
+  if (!(res0 < 1e140) || !(P.tolerance < 1e140) || !(P.rel_tol < 1e100)) return nan;
+  double t = 0.0;  // the smallest norm that is not converged
+  if (res0 > 0.0 && P.rel_tol > 0.0) {
+    if (!(res0 > 1e-140) || !(P.rel_tol > 1e-100)) return nan;
+    t = first_where(P.rel_tol * res0, [&](double r) { return !(r / res0 < P.rel_tol); });
+  }
+  if (P.tolerance > t) t = P.tolerance;
+  if (!(t > 0.0)) return t;  // 0 or NaN
+  if (!(t > 1e-140)) return nan;
+  return first_where(t * t, [&](double s) { return !(sqrt(s) < t); });
+}
+
+template <bool PREC>
+__global__ void __launch_bounds__(kBlock, kResidentPerSM)
+    pcg_resident_kernel(gbf_layout L, const double* __restrict__ coef,
+                        const double* __restrict__ diag, const double* __restrict__ pd,
+                        const double* __restrict__ b, double* __restrict__ x_io, TurnWord* z_all,
+                        TurnWord* slots, PcgState* st, double* hist, gbf_solve_params P) {
+  __shared__ double sh[16], ps[kBlock], bc[2], sent[2];
+  const int G = gridDim.x, n = L.n_cells, tid = threadIdx.x, blk = blockIdx.x;
+  const int c0 = blk * kBlock, c = c0 + tid;
+  const bool mine = c < n, lead = blk == 0 && tid == 0;
+  int* fault = &st->bar.fault;
+
+  // the cell's row: slot k at cell c + d[k] (bit k of `on`), inside the block (bit k of `in`)
+  double a[6] = {}, pn[6] = {}, dc = 0.0, pdc = 1.0, x = 0.0, r = 0.0, z = 0.0, p = 0.0;
+  int q[6] = {};
+  unsigned on = 0, in = 0;
+  if (mine) {
+    const int s = c >> 5, lane = c & 31, base = 192 * s + lane;
+    const int2* __restrict__ dm = reinterpret_cast<const int2*>(L.slot_dm) + 6 * s;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const int2 e = __ldg(dm + k);
+      a[k] = __ldg(coef + base + 32 * k);
+      if ((unsigned)e.y >> lane & 1u) {
+        on |= 1u << k;
+        q[k] = c + e.x;
+        if ((unsigned)(q[k] - c0) < (unsigned)kBlock) in |= 1u << k;
+      }
+    }
+    dc = __ldg(diag + c);
+    if (PREC) pdc = __ldg(pd + c);
+    x = x_io[c];
+  }
+  // (A v)[c] from v of the cell and of its neighbours: cell_amul_fixed's order
+  auto row = [&](double vc, const double (&v)[6]) {
+    double so = 0.0, sn = 0.0;
+    double t = first_term(__dmul_rn(a[0], v[0]));
+    so = (on & 1u) ? t : so;
+#pragma unroll
+    for (int k = 1; k < 3; ++k) {
+      t = __dadd_rn(so, __dmul_rn(a[k], v[k]));
+      so = (on >> k & 1u) ? t : so;
+    }
+    t = first_term(__dmul_rn(a[3], v[3]));
+    sn = (on & 8u) ? t : sn;
+#pragma unroll
+    for (int k = 4; k < 6; ++k) {
+      t = __dadd_rn(sn, __dmul_rn(a[k], v[k]));
+      sn = (on >> k & 1u) ? t : sn;
+    }
+    return __dadd_rn(__dadd_rn(__dmul_rn(dc, vc), so), sn);
+  };
+  long long wait = 1;  // number of the grid-wide wait
+  long long turn = 1;  // number of the z
+  bool ok = true;
+  auto z_of = [&](int q) { return z_all + (turn & 1) * (long long)n + q; };
+  auto publish_z = [&] {
+    if (mine) st_word(z_of(c), z, turn);
+  };
+  auto word = [&](int dest, int src, int which) {
+    return slots + (((size_t)dest * 2 + (wait & 1)) * 2 + which) * G + src;
+  };
+  // Publishes the block's sums (in thread 0, the second in thread 16)
+  auto publish = [&](double u, bool pair) {
+    if (tid == 0) sent[0] = u;
+    if (tid == 16) sent[1] = u;
+    __syncthreads();
+    for (int i = tid; i < G; i += kBlock) {
+      st_word(word(i, blk, 0), sent[0], wait);
+      if (pair) st_word(word(i, blk, 1), sent[1], wait);
+    }
+  };
+  // Two words polled together, as far as wanted: values into v0, v1.
+  auto poll_two = [&](const TurnWord* p0, bool want0, double& v0, const TurnWord* p1, bool want1,
+                      double& v1, long long number) {
+    long long polls = 0;
+    while (want0 || want1) {
+      TurnWord w0{0.0, 0}, w1{0.0, 0};
+      if (want0) w0 = ld_word(p0);
+      if (want1) w1 = ld_word(p1);
+      if (want0 && w0.turn == number) v0 = w0.v, want0 = false;
+      if (want1 && w1.turn == number) v1 = w1.v, want1 = false;
+      if ((want0 || want1) && !poll_again(polls, fault)) {
+        ok = false;
+        return;
+      }
+    }
+  };
+  // z of the neighbours in other blocks: slots 2 and 3 (the farthest ones of a
+  // mesh in cell order) first, which most threads want
+  auto gather = [&](double (&zq)[6]) {
+    const unsigned far = on & ~in;
+#pragma unroll
+    for (int k = 2; k >= 0; --k)
+      poll_two(z_of(q[k]), far >> k & 1u, zq[k], z_of(q[5 - k]), far >> (5 - k) & 1u, zq[5 - k],
+               turn);
+    ++turn;
+  };
+  // What this thread takes of all blocks' sums: those of blocks tid, tid + 256,
+  // ..., reduce_partials' order.
+  double got0 = 0.0, got1 = 0.0;
+  auto collect = [&](bool pair) {
+    got0 = got1 = 0.0;
+    for (int i = tid; i < G; i += kBlock) {
+      double w0 = 0.0, w1 = 0.0;
+      poll_two(word(blk, i, 0), true, w0, word(blk, i, 1), pair, w1, wait);
+      got0 = i == tid ? first_term(w0) : __dadd_rn(got0, w0);
+      if (pair) got1 = i == tid ? first_term(w1) : __dadd_rn(got1, w1);
+    }
+    ++wait;
+    return __syncthreads_and(ok) != 0;
+  };
+
+  // r = b - A x, z = M^-1 r, p = z
+  {
+    double v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = (on >> k & 1u) ? __ldcg(x_io + q[k]) : 0.0;
+    if (mine) {
+      r = __dsub_rn(__ldg(b + c), row(x, v));
+      z = PREC ? div_rn(r, pdc) : r;
+      p = z;
+    }
+  }
+  publish_z();
+  double u = block_sum_pair(mine ? __fma_rn(r, r, 0.0) : 0.0, mine ? __fma_rn(r, z, 0.0) : 0.0,
+                            sh, kBlock);
+  publish(u, true);
+  ps[tid] = p;
+  gather(pn);
+  if (!collect(true)) return;
+  u = block_sum_pair(got0, got1, sh, G);
+  if (tid == 0) bc[0] = u;
+  if (tid == 16) bc[1] = u;
+  __syncthreads();
+  double rr = bc[0], rzv = bc[1];
+  const double res0 = sqrt(rr);
+  const double limit = unconverged_rr(res0, P);  // NaN: apply the rules
+  auto converged = [&](double s, int iter) {
+    if (iter < P.min_iter) return false;
+    if (limit == limit && __double_as_longlong(s) >= 0) return less_nn(s, limit);
+    return monitor_converged(sqrt(s), res0, iter, P);
+  };
+  int iter = 1, n_hist = 1;
+  int status = converged(rr, 0) ? GBF_CONVERGED
+               : (P.max_iter < 1 ? GBF_MAX_ITER : GBF_RUNNING);
+  if (lead) hist[0] = res0;
+
+  for (int launched = 0; status == GBF_RUNNING && launched < P.max_iter; ++launched) {
+    double v[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = (in >> k & 1u) ? ps[q[k] - c0] : pn[k];
+    const double Ap = row(p, v);
+    u = block_sum_one(mine ? __fma_rn(p, Ap, 0.0) : 0.0, sh, kBlock);
+    publish(u, false);
+    // (the root of an earlier r.r, while the sums travel)
+    if (lead && launched > 0) hist[iter - 1] = sqrt_rn(rr);
+    if (!collect(false)) return;
+    u = block_sum_one(got0, sh, G);
+    if (tid == 0) bc[0] = u;
+    __syncthreads();
+    const double pAp = bc[0];
+    if (less_nn(fabs(pAp), 1e-30)) {
+      status = GBF_BREAKDOWN;  // pcg.py:153-156: x returned as is
+      break;
+    }
+    const double alpha = div_rn(rzv, pAp);
+    r = __dsub_rn(r, __dmul_rn(alpha, Ap));
+    z = (PREC && mine) ? div_rn(r, pdc) : r;
+    publish_z();
+    u = block_sum_pair(mine ? __fma_rn(r, r, 0.0) : 0.0, mine ? __fma_rn(r, z, 0.0) : 0.0, sh,
+                       kBlock);
+    publish(u, true);
+    x = __dadd_rn(x, __dmul_rn(alpha, p));
+    double zq[6] = {};
+    gather(zq);
+    if (!collect(true)) return;
+    u = block_sum_pair(got0, got1, sh, G);
+    if (tid == 0) bc[0] = u;
+    if (tid == 16) bc[1] = u;
+    __syncthreads();
+    const int it = iter;
+    rr = bc[0];
+    n_hist = it + 1;
+    if (converged(rr, it)) {
+      status = GBF_CONVERGED;
+      break;
+    }
+    const double beta = div_rn(bc[1], rzv);
+    rzv = bc[1];
+    iter = it + 1;
+    if (it >= P.max_iter) {
+      status = GBF_MAX_ITER;
+      break;
+    }
+    p = __dadd_rn(z, __dmul_rn(beta, p));
+    ps[tid] = p;
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      if ((on & ~in) >> k & 1u) pn[k] = __dadd_rn(zq[k], __dmul_rn(beta, pn[k]));
+    __syncthreads();
+  }
+  if (mine) x_io[c] = x;
+  if (lead) {
+    if (n_hist > 1) hist[n_hist - 1] = sqrt_rn(rr);
+    st->status = status;
+    st->res = sqrt_rn(rr);
+    st->res0 = res0;
+    st->n_hist = n_hist;
+    st->iter = iter;
+    st->rz = rzv;
+  }
+}
+
 // Blocks of the single-launch PCG that can be resident at once (0 if the
 // device cannot launch it cooperatively).
 template <int KIND, bool PREC>
@@ -328,6 +706,7 @@ static int persistent_grid(int n) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_persistent_kernel<KIND, PREC>,
                                                     kBlock, 0) != cudaSuccess || per_sm <= 0)
     return 0;
+  if (per_sm > kPersistentPerSM<KIND, PREC>) per_sm = kPersistentPerSM<KIND, PREC>;
   long long g = (long long)per_sm * sms;
   const long long need = (n + kBlock - 1) / kBlock;
   if (g > need) g = need;
@@ -351,16 +730,44 @@ static cudaError_t launch_persistent(int grid, const gbf_layout* L, const double
 // variant 0 (above it the per-iteration launch cost is negligible).
 constexpr int kPersistentMaxCells = 1 << 21;
 
+// Whether pcg_resident_kernel takes the system: a hex 3+3 layout, one cell a
+// resident thread.
+template <bool PREC>
+static bool resident_fits(const gbf_layout& L, bool hex) {
+  int dev = 0, coop = 0, sms = 0, per_sm = 0;
+  if (!hex || cudaGetDevice(&dev) != cudaSuccess) return false;
+  cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!coop || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_resident_kernel<PREC>,
+                                                             kBlock, 0) != cudaSuccess)
+    return false;
+  if (per_sm > kResidentPerSM) per_sm = kResidentPerSM;
+  if (L.n_cells > (long long)kResidentMaxBlocks * kBlock) return false;
+  return L.n_cells <= (long long)per_sm * sms * kBlock;
+}
+
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 }  // namespace gbf
 
 using namespace gbf;
 
-extern "C" size_t gbf_pcg_workspace_bytes(int32_t n) {
-  if (n < 0) return 0;
+// r, z, p, Ap, the partial sums and the state.
+static size_t pcg_base_bytes(int n) {
   return 4 * align256(sizeof(double) * (size_t)n) + align256(sizeof(double) * 2 * kMaxGrid) +
          align256(sizeof(PcgState));
+}
+
+// Sum words of pcg_resident_kernel on G blocks.
+static size_t resident_words(int G) {
+  return (size_t)G * 2 * kSlotSets * G;
+}
+
+extern "C" size_t gbf_pcg_workspace_bytes(int32_t n) {
+  if (n < 0) return 0;
+  const long long G = ((long long)n + kBlock - 1) / kBlock;
+  return pcg_base_bytes(n) +
+         (G <= kResidentMaxBlocks ? align256(resident_words((int)G) * sizeof(TurnWord)) : 0);
 }
 
 extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const double* diag,
@@ -402,13 +809,28 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
   // single launch (variant 2, or variant 0 on a launch-bound system)
   if (P->variant == 2 || (P->variant == 0 && n <= kPersistentMaxCells)) {
     const bool hex = layout_kind(*L) == kLayoutHex33;
-    const int Gp = hex ? (pd ? persistent_grid<kLayoutHex33, true>(n)
+    const bool resident = pd ? resident_fits<true>(*L, hex) : resident_fits<false>(*L, hex);
+    const int Gp = resident ? (n + kBlock - 1) / kBlock
+                   : hex ? (pd ? persistent_grid<kLayoutHex33, true>(n)
                              : persistent_grid<kLayoutHex33, false>(n))
                        : (pd ? persistent_grid<kLayoutGeneric, true>(n)
                              : persistent_grid<kLayoutGeneric, false>(n));
     if (Gp > 0) {
       cudaError_t e;
-      if (hex)
+      if (resident) {
+        // z words over r, z, p, Ap (32 bytes a cell), sum words behind
+        TurnWord* zw = reinterpret_cast<TurnWord*>(w);
+        TurnWord* sw = reinterpret_cast<TurnWord*>(w + pcg_base_bytes(n));
+        GBF_CHECK_CUDA(cudaMemsetAsync(zw, 0, 2 * sizeof(TurnWord) * (size_t)n, s));
+        GBF_CHECK_CUDA(cudaMemsetAsync(sw, 0, resident_words(Gp) * sizeof(TurnWord), s));
+        gbf_layout Lc = *L;
+        gbf_solve_params Pc = *P;
+        void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&pd, (void*)&b, &x, &zw, &sw,
+                        &v.st, &hist, &Pc};
+        e = cudaLaunchCooperativeKernel(pd ? (const void*)pcg_resident_kernel<true>
+                                           : (const void*)pcg_resident_kernel<false>,
+                                        dim3(Gp), dim3(kBlock), args, 0, s);
+      } else if (hex)
         e = pd ? launch_persistent<kLayoutHex33, true>(Gp, L, coef, diag, pd, b, x, v, hist, P, s)
                : launch_persistent<kLayoutHex33, false>(Gp, L, coef, diag, pd, b, x, v, hist, P,
                                                         s);
