@@ -46,8 +46,10 @@ __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q,
   if (D.mode == 1) return __ldg(D.face + f);
   const double dp = cell_D(D, p);
   if (!internal) return dp;
-  const double w = __ldg(D.w + f);
-  return __dadd_rn(__dmul_rn(w, dp), __dmul_rn(__dsub_rn(1.0, w), cell_D(D, q)));
+  const double w = __ldg(D.w + f), v = __dsub_rn(1.0, w), dq = cell_D(D, q);
+  // mode 3 divides twice on the integer pipe; mode 2 leaves it room for the products
+  if (D.mode == 2) return __dadd_rn(mul_int(w, dp), mul_int(v, dq));
+  return __dadd_rn(__dmul_rn(w, dp), __dmul_rn(v, dq));
 }
 
 // (0 + sum over the cell's owner-side faces) + (sum over its neighbour-side
@@ -445,8 +447,8 @@ __global__ void __launch_bounds__(kBlock)
       if (f < 0) continue;
       const int q = __ldg(L.slot_col + i);
       double fl = __dmul_rn(face_D(D, f, c, q, true), __dsub_rn(__ldg(phi + q), pc));
-      fl = __dmul_rn(fl, face_smag(areas + 3 * (size_t)f));
-      fl = __dmul_rn(fl, __ldg(delta + f));
+      fl = mul_int(fl, face_smag(areas + 3 * (size_t)f));
+      fl = mul_int(fl, __ldg(delta + f));
       so = __dadd_rn(so, fl);
     }
     for (int k = 0; k < cs.wn; ++k) {
@@ -455,8 +457,8 @@ __global__ void __launch_bounds__(kBlock)
       if (f < 0) continue;
       const int p = __ldg(L.slot_col + i);
       double fl = __dmul_rn(face_D(D, f, p, c, true), __dsub_rn(pc, __ldg(phi + p)));
-      fl = __dmul_rn(fl, face_smag(areas + 3 * (size_t)f));
-      fl = __dmul_rn(fl, __ldg(delta + f));
+      fl = mul_int(fl, face_smag(areas + 3 * (size_t)f));
+      fl = mul_int(fl, __ldg(delta + f));
       sn = __dadd_rn(sn, -fl);
     }
   }

@@ -29,6 +29,11 @@ __device__ __forceinline__ double lerp_w(double w, double a, double b) {
   return __dadd_rn(__dmul_rn(w, a), __dmul_rn(__dsub_rn(1.0, w), b));
 }
 
+// The same with both products on the integer pipe.
+__device__ __forceinline__ double lerp_int(double w, double v, double a, double b) {
+  return __dadd_rn(mul_int(w, a), mul_int(v, b));  // v = 1 - w
+}
+
 __device__ __forceinline__ double fma_norm3(const double* __restrict__ a) {
   const double x = __ldg(a), y = __ldg(a + 1), z = __ldg(a + 2);
   return sqrt_rn(__fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
@@ -61,10 +66,9 @@ __device__ __forceinline__ double rc_term(int f, const int32_t* __restrict__ own
                                           const double* __restrict__ w) {
   const int P = __ldg(own + f), N = __ldg(nei + f);
   const double wf = w ? __ldg(w + f) : 0.5;
-  const double ia = lerp_w(wf, __ldg(inv_A + P), __ldg(inv_A + N));
+  const double ia = lerp_int(wf, __dsub_rn(1.0, wf), __ldg(inv_A + P), __ldg(inv_A + N));
   const double dp = __dsub_rn(__ldg(p + P), __ldg(p + N));
-  return __dmul_rn(__dmul_rn(__dmul_rn(ia, dp), fma_norm3(areas + 3 * (size_t)f)),
-                   __ldg(delta + f));
+  return __dmul_rn(mul_int(mul_int(ia, dp), fma_norm3(areas + 3 * (size_t)f)), __ldg(delta + f));
 }
 
 // phi_f = (w HbyA_P + (1-w) HbyA_N) . S_f on internal faces, HbyA_P . S_f on
@@ -82,10 +86,11 @@ __global__ void __launch_bounds__(kBlock)
   double s;
   if (f < nint) {
     const int N = __ldg(nei + f);
-    const double wf = w ? __ldg(w + f) : 0.5;
+    const double wf = w ? __ldg(w + f) : 0.5, vf = __dsub_rn(1.0, wf);
     for (int k = 0; k < 3; ++k) {
-      const double hf = lerp_w(wf, __ldg(HbyA + 3 * (size_t)P + k), __ldg(HbyA + 3 * (size_t)N + k));
-      const double t = __dmul_rn(hf, __ldg(areas + 3 * (size_t)f + k));
+      const double hf =
+          lerp_int(wf, vf, __ldg(HbyA + 3 * (size_t)P + k), __ldg(HbyA + 3 * (size_t)N + k));
+      const double t = mul_int(hf, __ldg(areas + 3 * (size_t)f + k));
       s = k == 0 ? first_term(t) : __dadd_rn(s, t);
     }
     if (p) s = __dadd_rn(s, rc_term(f, own, nei, p, A, areas, delta, w));
@@ -151,10 +156,12 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           if (f[j] < 0) continue;
-          const double pf = side == 0 ? lerp_w(wf[j], pc, pn[j]) : lerp_w(wf[j], pn[j], pc);
+          const double vf = __dsub_rn(1.0, wf[j]);
+          const double pf = side == 0 ? lerp_int(wf[j], vf, pc, pn[j])
+                                      : lerp_int(wf[j], vf, pn[j], pc);
           const double pfs = side == 0 ? pf : -pf;  // a sign commutes with the rounding
           for (int q = 0; q < 3; ++q) {
-            const double t = __dmul_rn(pfs, __ldg(areas + 3 * (size_t)f[j] + q));
+            const double t = mul_int(pfs, __ldg(areas + 3 * (size_t)f[j] + q));
             g[q] = first ? first_term(t) : __dadd_rn(g[q], t);
           }
           first = false;

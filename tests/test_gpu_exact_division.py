@@ -1,4 +1,4 @@
-"""The integer-pipe division and square root (csrc/exact.cuh) against numpy's IEEE
+"""The integer-pipe product, division and square root (csrc/exact.cuh) against numpy's IEEE
 operations, bit for bit, through the operators that divide and take roots
 directly: compute_HbyA (H / max(|A|, 1e-30)) and fvm.laplacian's lower
 coefficient on unit volumes and deltas (-|S_f|)."""
@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from pyopenfoam_gb300.discretisation import fvm
-from pyopenfoam_gb300.solvers.rhie_chow import compute_HbyA
+from pyopenfoam_gb300.solvers.rhie_chow import compute_face_flux_HbyA, compute_HbyA
 
 pytestmark = pytest.mark.gpu
 N = 1 << 16
@@ -91,3 +91,21 @@ def test_square_root_is_ieee(scale, odd):
     with np.errstate(all="ignore"):
         want = -np.sqrt(x * x + y * y)
     assert same(A.lower.cpu().numpy(), want) and same(A.upper.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kind", ["random", "near_midpoint", "exact_and_close", "special"])
+def test_product_is_ieee(kind):
+    """The integer-pipe product, through compute_face_flux_HbyA: the flux of a boundary face with
+    area (s, 0, 0) is h s (+ 0 + 0); of an internal one with weight 1, (1 h + 0 h') s."""
+    a, b = pairs(kind, np.random.default_rng(9))
+    n = a.shape[0]
+    H = torch.as_tensor(np.stack([np.concatenate([a, [1.0]])] + [np.ones(n + 1)] * 2, 1)).cuda()
+    S = torch.as_tensor(np.stack([b, np.zeros(n), np.zeros(n)], 1)).cuda()
+    own = torch.arange(n).cuda()
+    with np.errstate(all="ignore"):
+        want = a * b + 0.0
+        inner = (1.0 * a + 0.0 * np.concatenate([a[1:], [1.0]])) * b + 0.0
+    got = compute_face_flux_HbyA(H, S, own, own + 1, n, torch.ones(n, dtype=torch.float64).cuda())
+    assert same(got.cpu().numpy(), inner)
+    got = compute_face_flux_HbyA(H, S, own, own[:0], 0)
+    assert same(got.cpu().numpy(), want)
