@@ -32,6 +32,25 @@ class FvMatrix(LduMatrix):
         self._field_old: torch.Tensor | None = None
         self._relaxation_factor: float = 1.0
 
+    @classmethod
+    def _assembled(cls, n_cells: int, owner: torch.Tensor, neighbour: torch.Tensor,
+                   topology, diag: torch.Tensor, lower: torch.Tensor, upper: torch.Tensor,
+                   source: torch.Tensor | None = None) -> "FvMatrix":
+        """A float64 matrix on checked addressing (contiguous int64, its
+        ``topology`` at hand) that takes the given arrays: the constructor clears
+        four it then drops (8 launches and 2.2 us each of the 200 us that
+        assembling the two operators of a 500 000-cell momentum equation takes)."""
+        m = cls.__new__(cls)
+        m._device, m._dtype = topology.device, torch.float64
+        m._n_cells, m._n_internal_faces = int(n_cells), int(neighbour.shape[0])
+        m._owner, m._neighbour = owner, neighbour
+        m._diag, m._lower, m._upper = diag, lower, upper
+        m._csr_cache, m._topology = {}, topology
+        m._source = (torch.zeros(n_cells, device=m._device, dtype=torch.float64) if source is None
+                     else source)
+        m._field_old, m._relaxation_factor = None, 1.0
+        return m
+
     @property
     def source(self) -> torch.Tensor:
         return self._source

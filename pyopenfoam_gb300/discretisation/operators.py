@@ -47,8 +47,8 @@ class MeshData:
         nei = mesh.neighbour.to(self.device)
         if own.shape[0] != self.n_faces or nei.shape[0] != self.n_internal:
             raise ValueError("mesh owner/neighbour sizes do not match n_faces/n_internal_faces")
-        self.owner = own[: self.n_internal].to(torch.int64)
-        self.neighbour = nei.to(torch.int64)
+        self.owner = own[: self.n_internal].to(torch.int64).contiguous()
+        self.neighbour = nei.to(torch.int64).contiguous()
         self.owner_all32 = own.to(torch.int32).contiguous()
         own_b = own[self.n_internal:].to("cpu", torch.int32).numpy()
         ptr = np.empty(self.n_cells + 1, np.int32)
@@ -102,10 +102,11 @@ def _resolve_mesh(phi: Any, mesh: Any):
     return mesh
 
 
-def _make_fvmatrix(md: MeshData) -> FvMatrix:
-    """FvMatrix on the mesh's internal-face addressing
-    (operators.py:205-213)."""
-    return FvMatrix(md.n_cells, md.owner, md.neighbour, device=md.device, dtype=torch.float64)
+def _make_fvmatrix(md: MeshData, topo, lower: torch.Tensor, upper: torch.Tensor, diag: torch.Tensor,
+                   source: torch.Tensor | None = None) -> FvMatrix:
+    """FvMatrix on the mesh's internal-face addressing with the assembled
+    coefficients (operators.py:205-213)."""
+    return FvMatrix._assembled(md.n_cells, md.owner, md.neighbour, topo, diag, lower, upper, source)
 
 
 class _LaplacianCoeffs(torch.autograd.Function):
@@ -163,8 +164,7 @@ class fvm:  # noqa: N801 -- the reference's name
         grad makes the returned coefficients differentiable."""
         mesh = _resolve_mesh(phi, mesh)
         md = mesh_data(mesh)
-        mat = _make_fvmatrix(md)
-        topo = mat.topology()
+        topo = md.topology()
         areas = md.field("face_areas")
         delta = md.field("delta_coefficients")
         volumes = md.field("cell_volumes")
@@ -195,8 +195,7 @@ class fvm:  # noqa: N801 -- the reference's name
             lower, upper, diag = _assemble(md, topo, areas, delta, volumes, mode, value,
                                            None if d_face is None else d_face.detach().contiguous(),
                                            d_cell, w)
-        mat._lower, mat._upper, mat._diag = lower, upper, diag
-        return mat
+        return _make_fvmatrix(md, topo, lower, upper, diag)
 
     @staticmethod
     def div(phi: Any, U: Any, scheme: str = "Gauss upwind", *, mesh: Any = None) -> FvMatrix:
@@ -214,8 +213,7 @@ class fvm:  # noqa: N801 -- the reference's name
         flux = phi.internal_field if hasattr(phi, "internal_field") else phi
         flux = torch.as_tensor(flux).to(device=md.device, dtype=torch.float64)
         flux = flux[: md.n_internal].contiguous()
-        mat = _make_fvmatrix(md)
-        topo = mat.topology()
+        topo = md.topology()
         volumes = md.field("cell_volumes")
         dev = md.device
         lower = torch.empty(max(md.n_internal, 1), device=dev, dtype=torch.float64)
@@ -224,6 +222,5 @@ class fvm:  # noqa: N801 -- the reference's name
         _lib.check(_lib.lib().gbf_div_upwind_assemble_f64(
             topo.layout_ref, flux.data_ptr(), volumes.data_ptr(), lower.data_ptr(),
             upper.data_ptr(), diag.data_ptr(), _lib.stream_ptr(dev)), "gbf_div_upwind_assemble_f64")
-        mat._lower, mat._upper, mat._diag = (lower[: md.n_internal], upper[: md.n_internal],
-                                             diag[: md.n_cells])
-        return mat
+        return _make_fvmatrix(md, topo, lower[: md.n_internal], upper[: md.n_internal],
+                              diag[: md.n_cells])

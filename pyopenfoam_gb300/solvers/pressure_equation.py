@@ -48,8 +48,7 @@ def assemble_pressure_equation(phiHbyA: torch.Tensor, A_p: torch.Tensor, mesh: A
                                face_weights: torch.Tensor | None = None) -> FvMatrix:
     md = mesh_data(mesh)
     dev = md.device
-    mat = _make_fvmatrix(md)
-    topo = mat.topology()
+    topo = md.topology()
     if face_weights is None:
         face_weights = getattr(mesh, "face_weights", None)
     w = md.weights(topo) if face_weights is None else face_weights
@@ -71,9 +70,7 @@ def assemble_pressure_equation(phiHbyA: torch.Tensor, A_p: torch.Tensor, mesh: A
         w.data_ptr(), A.data_ptr(), md.field("cell_volumes").data_ptr(), phi.data_ptr(),
         lower.data_ptr(), upper.data_ptr(), diag.data_ptr(), source.data_ptr(),
         _lib.stream_ptr(dev)), "gbf_pressure_assemble_f64")
-    mat._lower, mat._upper, mat._diag = lower[:nint], upper[:nint], diag[:n]
-    mat.source = source[:n]
-    return mat
+    return _make_fvmatrix(md, topo, lower[:nint], upper[:nint], diag[:n], source[:n])
 
 
 def solve_pressure_equation(p_eqn: FvMatrix, p: torch.Tensor, solver: LinearSolverBase,
