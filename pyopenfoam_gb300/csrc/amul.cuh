@@ -9,6 +9,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
@@ -21,6 +22,32 @@ __device__ __forceinline__ T ldx(const T* p) {
     return __ldcg(p);
   else
     return __ldg(p);
+}
+
+// Product of the fixed-width gather's slot K.  In FP64 that gather is bound by
+// the FP64 pipe (13 operations a hex cell, of which six additions must run
+// there), so most of its products run on the integer pipe beside it: of a hex
+// cell's seven the five for which this is true, 8 x 64 against 5 x 80 clocks a
+// warp (Amul of 256^3 437 -> 296 us, of 128^3 59.5 -> 43.6 us).  Slots that hold
+// no face carry 1 x 1, so that a zero does not take the warp through the
+// product's slow path.  The general gather keeps plain products: it waits for
+// its columns and x, and the integer code's registers cost it occupancy (128^3
+// under a random numbering 119 -> 162 us).
+template <int K>
+constexpr bool kIntProduct = K % 3 != 0 || K == 3;
+
+template <int K>
+__device__ __forceinline__ double slot_mul(double a, double x) {
+  if constexpr (kIntProduct<K>)
+    return mul_int(a, x);
+  else
+    return mul_rn(a, x);
+}
+
+template <int W, typename T, int... K>
+__device__ __forceinline__ void slot_products(T (&p)[W], const T (&a)[W], const T (&x)[W],
+                                              std::integer_sequence<int, K...>) {
+  ((p[K] = slot_mul<K>(a[K], x[K])), ...);
 }
 
 // Sum over `cnt` slots starting at slot k0 of cell c (slot index i0 =
@@ -83,15 +110,20 @@ __device__ __forceinline__ A cell_amul(const gbf_layout& L, const T* __restrict_
         a[4 + k] = (k < cs.wn) ? __ldg(coef + cs.base + 32 * (cs.wo + k)) : (T)0;
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) xv[k] = (col[k] >= 0) ? ldx<COH>(x + col[k]) : (T)0;
-      if (col[0] >= 0) so = first_term((A)mul_rn(a[0], xv[0]));
+      for (int k = 0; k < 8; ++k) {
+        xv[k] = (col[k] >= 0) ? ldx<COH>(x + col[k]) : (T)0;
+      }
+      T p[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) p[k] = mul_rn(a[k], xv[k]);
+      if (col[0] >= 0) so = first_term((A)p[0]);
 #pragma unroll
       for (int k = 1; k < 4; ++k)
-        if (col[k] >= 0) so = add_rn(so, (A)mul_rn(a[k], xv[k]));
-      if (col[4] >= 0) sn = first_term((A)mul_rn(a[4], xv[4]));
+        if (col[k] >= 0) so = add_rn(so, (A)p[k]);
+      if (col[4] >= 0) sn = first_term((A)p[4]);
 #pragma unroll
       for (int k = 5; k < 8; ++k)
-        if (col[k] >= 0) sn = add_rn(sn, (A)mul_rn(a[k], xv[k]));
+        if (col[k] >= 0) sn = add_rn(sn, (A)p[k]);
     } else {
       so = slot_sum<T, A, COH>(L, coef, x, c, cs.base, cs.e0, cs.wo);
       sn = slot_sum<T, A, COH>(L, coef, x, c, cs.base + 32 * cs.wo, cs.e0 + cs.wo, cs.wn);
@@ -147,17 +179,32 @@ __device__ __forceinline__ A cell_amul_fixed(const gbf_layout& L, const T* __res
 #pragma unroll
   for (int k = 0; k < W; ++k) {
     on[k] = (m[k] >> lane) & 1u;
-    xv[k] = on[k] ? ldx<COH>(x + c + d[k]) : (T)0;
+    xv[k] = on[k] ? ldx<COH>(x + c + d[k]) : (T)(sizeof(T) == 8 ? 1 : 0);
   }
   A so = (A)0, sn = (A)0;
-  if (WO > 0 && on[0]) so = first_term((A)mul_rn(a[0], xv[0]));
+  if constexpr (sizeof(T) == 8) {
+    T p[W];
 #pragma unroll
-  for (int k = 1; k < WO; ++k)
-    if (on[k]) so = add_rn(so, (A)mul_rn(a[k], xv[k]));
-  if (WN > 0 && on[WO]) sn = first_term((A)mul_rn(a[WO], xv[WO]));
+    for (int k = 0; k < W; ++k) a[k] = on[k] ? a[k] : (T)1;
+    slot_products<W>(p, a, xv, std::make_integer_sequence<int, W>());
+    if (WO > 0 && on[0]) so = first_term(p[0]);
 #pragma unroll
-  for (int k = WO + 1; k < W; ++k)
-    if (on[k]) sn = add_rn(sn, (A)mul_rn(a[k], xv[k]));
+    for (int k = 1; k < WO; ++k)
+      if (on[k]) so = add_rn(so, p[k]);
+    if (WN > 0 && on[WO]) sn = first_term(p[WO]);
+#pragma unroll
+    for (int k = WO + 1; k < W; ++k)
+      if (on[k]) sn = add_rn(sn, p[k]);
+  } else {
+    if (WO > 0 && on[0]) so = first_term((A)mul_rn(a[0], xv[0]));
+#pragma unroll
+    for (int k = 1; k < WO; ++k)
+      if (on[k]) so = add_rn(so, (A)mul_rn(a[k], xv[k]));
+    if (WN > 0 && on[WO]) sn = first_term((A)mul_rn(a[WO], xv[WO]));
+#pragma unroll
+    for (int k = WO + 1; k < W; ++k)
+      if (on[k]) sn = add_rn(sn, (A)mul_rn(a[k], xv[k]));
+  }
   A y = (A)mul_rn(__ldg(diag + c), xc);
   if (NEI_FIRST) {
     y = add_rn(y, sn);
