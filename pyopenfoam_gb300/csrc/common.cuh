@@ -242,6 +242,37 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
   return t;
 }
 
+// Both block_sum(a) and block_sum(b), for blocks of kBlock threads, valid in
+// thread 0: lanes 0-15 of a warp carry a, lanes 16-31 b, so each level of the
+// two trees is one addition (an FP64 instruction takes 64 clocks of its SM
+// quarter on GB300, and a kernel with one cell a thread spends more of them on
+// its sums than on its cells).  `sh` holds 2 * kBlock / 32.
+struct SumPair {
+  double a, b;
+};
+__device__ __forceinline__ SumPair block_sum_two(double a, double b, double* sh) {
+  static_assert(kBlock == 256, "eight warps");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool low = lane < 16;
+  double v = (low ? a : b) + __shfl_xor_sync(0xffffffffu, low ? b : a, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
+  __syncthreads();  // sh may still be read by a previous call
+  if ((lane & 15) == 0) sh[(low ? 0 : 8) + wid] = v;
+  __syncthreads();
+  SumPair s{0.0, 0.0};
+  if (wid == 0) {
+    // block_sum's tree over 32 entries first adds zeros: -0.0 becomes +0.0
+    v = (lane & 15) < 8 ? sh[(low ? 0 : 8) + (lane & 7)] : 0.0;
+    if (__double_as_longlong(v) == (long long)0x8000000000000000ULL) v = 0.0;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
+    s.b = __shfl_sync(0xffffffffu, v, 16);
+    s.a = v;
+  }
+  return s;
+}
+
 // Returns true in every thread of the block that finished last.  The caller
 // wrote its partials (thread 0) before calling; the last block reads only
 // partials (and state written by earlier kernels), so only thread 0 fences
@@ -283,6 +314,34 @@ __device__ __forceinline__ T reduce_partials(const T* partials, int n, T* sh) {
       if (i0 + u * B < n) v += q[u];
   }
   return block_sum(v, sh);
+}
+
+// reduce_partials of two rows of n partials, results in thread 0.  Four rows
+// at a time: with eight, the kernels that end in it take 64 registers instead
+// of 40 and the PBiCGStab solves were 4 % slower.
+__device__ __forceinline__ SumPair reduce_partials_two(const double* pa, const double* pb, int n,
+                                                       double* sh) {
+  constexpr int U = 4;
+  const int B = blockDim.x;
+  const int lane = threadIdx.x & 31;
+  double va = 0.0, vb = 0.0;
+  for (int w0 = threadIdx.x - lane; w0 < n; w0 += U * B) {  // by warps
+    const int i0 = w0 + lane;
+    double qa[U], qb[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      qa[u] = (i0 + u * B < n) ? __ldcg(pa + i0 + u * B) : 0.0;
+      qb[u] = (i0 + u * B < n) ? __ldcg(pb + i0 + u * B) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (w0 + u * B < n) {  // no addition for nothing; a lane past the end adds 0.0
+        va += qa[u];
+        vb += qb[u];
+      }
+    }
+  }
+  return block_sum_two(va, vb, sh);
 }
 
 // 0.0 + p without a floating-point add: p itself, except that -0.0 becomes

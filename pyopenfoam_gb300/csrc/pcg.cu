@@ -18,6 +18,13 @@
 // Element-wise arithmetic rounds exactly as the reference's torch ops
 // (alpha*p rounded, then added; r / d by IEEE division); dot products are
 // deterministic fixed-order trees with fused multiply-add accumulation.
+//
+// K_update is bound by the FP64 pipe (64 clocks of its SM quarter an
+// instruction), so alpha p and the division run on the integer pipe
+// (exact.cuh, the same bits; not alpha Ap as well: the two pipes are then
+// about even) and r.r and r.z share one tree.  Whole solves with DIC, before
+// and after: 120x110x100 72.2 -> 60.4 ms, 170x160x150 249.5 -> 173.1 ms,
+// 90x80x70 in no order 47.7 -> 39.2 ms (732, 926 and 553 iterations).
 #include <math.h>
 #include <string.h>
 
@@ -53,7 +60,7 @@ __global__ void __launch_bounds__(kBlock)
     pcg_init_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
                     const double* __restrict__ pd, const double* __restrict__ b,
                     const double* __restrict__ x, PcgVecs v, double* hist, gbf_solve_params P) {
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   double rr = 0.0, rz = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += G * blockDim.x) {
@@ -66,15 +73,14 @@ __global__ void __launch_bounds__(kBlock)
     rr = fma(rc, rc, rr);
     rz = fma(rc, zc, rz);
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two(rr, rz, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = rr;
-    v.partials[G + blockIdx.x] = rz;
+    v.partials[blockIdx.x] = sums.a;
+    v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[0])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trz = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
       PcgState* st = v.st;
       const double res = sqrt(trr);
@@ -97,7 +103,7 @@ __global__ void __launch_bounds__(kBlock)
     pcg_ap_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
                   PcgVecs v) {
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   const double* p = v.p;
   double acc = 0.0;
@@ -127,12 +133,12 @@ __global__ void __launch_bounds__(kBlock)
     pcg_update_kernel(int n, const double* __restrict__ pd, double* __restrict__ x, PcgVecs v,
                       double* hist, gbf_solve_params P) {
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   const double alpha = v.st->alpha;
   double rr = 0.0, rz = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += G * blockDim.x) {
-    const double xc = __dadd_rn(x[c], __dmul_rn(alpha, v.p[c]));
+    const double xc = __dadd_rn(x[c], mul_int(alpha, v.p[c]));
     const double rc = __dsub_rn(v.r[c], __dmul_rn(alpha, v.Ap[c]));
     const double zc = PREC ? div_rn(rc, __ldg(pd + c)) : rc;
     x[c] = xc;
@@ -141,15 +147,14 @@ __global__ void __launch_bounds__(kBlock)
     rr = fma(rc, rc, rr);
     rz = fma(rc, zc, rz);
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two(rr, rz, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = rr;
-    v.partials[G + blockIdx.x] = rz;
+    v.partials[blockIdx.x] = sums.a;
+    v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[2])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trz = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
       PcgState* st = v.st;
       const int it = st->iter;
@@ -203,7 +208,7 @@ __global__ void __launch_bounds__(kBlock, (kPersistentPerSM<KIND, PREC>))
                           const double* __restrict__ diag, const double* __restrict__ pd,
                           const double* __restrict__ b, double* __restrict__ x, PcgVecs v,
                           double* hist, gbf_solve_params P) {
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x, n = L.n_cells;
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x, cs = G * blockDim.x;
   const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
@@ -224,19 +229,17 @@ __global__ void __launch_bounds__(kBlock, (kPersistentPerSM<KIND, PREC>))
     rr = fma(rc, rc, rr);
     rz = fma(rc, zc, rz);
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two(rr, rz, sh);
   if (threadIdx.x == 0) {
-    partB[blockIdx.x] = rr;
-    partB[G + blockIdx.x] = rz;
+    partB[blockIdx.x] = sums.a;
+    partB[G + blockIdx.x] = sums.b;
   }
   if (!grid_barrier(bar, G)) return;
-  double s0 = reduce_partials(partB, G, sh);
-  double s1 = reduce_partials(partB + G, G, sh);
+  SumPair total = reduce_partials_two(partB, partB + G, G, sh);
   __shared__ double bc[2];
   if (threadIdx.x == 0) {
-    bc[0] = s0;
-    bc[1] = s1;
+    bc[0] = total.a;
+    bc[1] = total.b;
   }
   __syncthreads();
   const double res0 = sqrt(bc[0]);
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kBlock, (kPersistentPerSM<KIND, PREC>))
     acc = block_sum(acc, sh);
     if (threadIdx.x == 0) partA[blockIdx.x] = acc;
     if (!grid_barrier(bar, G)) return;
-    s0 = reduce_partials(partA, G, sh);
+    const double s0 = reduce_partials(partA, G, sh);
     if (threadIdx.x == 0) bc[0] = s0;
     __syncthreads();
     const double pAp = bc[0];
@@ -280,18 +283,16 @@ __global__ void __launch_bounds__(kBlock, (kPersistentPerSM<KIND, PREC>))
       rr = fma(rc, rc, rr);
       rz = fma(rc, zc, rz);
     }
-    rr = block_sum(rr, sh);
-    rz = block_sum(rz, sh);
+    const SumPair sums = block_sum_two(rr, rz, sh);
     if (threadIdx.x == 0) {
-      partB[blockIdx.x] = rr;
-      partB[G + blockIdx.x] = rz;
+      partB[blockIdx.x] = sums.a;
+      partB[G + blockIdx.x] = sums.b;
     }
     if (!grid_barrier(bar, G)) return;
-    s0 = reduce_partials(partB, G, sh);
-    s1 = reduce_partials(partB + G, G, sh);
+    total = reduce_partials_two(partB, partB + G, G, sh);
     if (threadIdx.x == 0) {
-      bc[0] = s0;
-      bc[1] = s1;
+      bc[0] = total.a;
+      bc[1] = total.b;
     }
     __syncthreads();
     const int it = iter;
