@@ -222,6 +222,12 @@ __device__ __forceinline__ bool above(double a, double t) {
 }
 __device__ __forceinline__ bool above_tiny(double a) { return above(a, 1e-30); }
 
+// a >= t for a >= 0 or NaN (false for NaN) and a positive constant t.
+__device__ __forceinline__ bool at_least(double a, double t) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+  return b >= (unsigned long long)__double_as_longlong(t) && b <= 0x7ff0000000000000ull;
+}
+
 // max(|a|, 1e-30), 1e-30 for NaN.
 __device__ __forceinline__ double max_abs_tiny(double a) {
   const double m = fabs(a);
