@@ -680,6 +680,17 @@ int gbf_face_geometry_f64(int32_t n_faces, const int32_t* face_ptr, const int32_
  * cell_faces_h n_faces + n_internal.                                       */
 int gbf_cell_faces(int32_t n_cells, int32_t n_faces, int32_t n_internal, const int32_t* owner_h,
                    const int32_t* neighbour_h, int32_t* cell_ptr_h, int32_t* cell_faces_h);
+/* The same lists made on the device, with 32-bit copies of owner and
+ * neighbour (int64, DEVICE).  work holds gbf_cell_faces_work_ints int32.
+ * status (two DEVICE uint32): [0] the lowest face with a cell outside
+ * [0, n_cells), 0xffffffff if none; [1] the bitwise complement of the largest
+ * number of faces of a cell.  The lists are valid if [0] is 0xffffffff and no
+ * cell has more than 4096 faces.  n_cells and n_faces at least 1.           */
+int64_t gbf_cell_faces_work_ints(int32_t n_cells, int32_t n_faces, int32_t n_internal);
+int gbf_cell_faces_device(int32_t n_cells, int32_t n_faces, int32_t n_internal,
+                          const int64_t* owner, const int64_t* neighbour, int32_t* owner32,
+                          int32_t* neighbour32, int32_t* cell_ptr, int32_t* cell_faces,
+                          int32_t* work, uint32_t* status, void* stream);
 /* Cell volumes [n_cells] and centres [n_cells][3] by the tet decomposition
  * about the mean of the cell's distinct vertices (mesh_geometry.py:139-254;
  * the mean is taken in ascending vertex order).  *status (a DEVICE int32,

@@ -178,6 +178,9 @@ EXPORTED: dict[str, tuple] = {
     "gbf_boundary_flux_sum_f64": (ctypes.c_int, [_c_i32, _c_i32, _c_vp, _c_vp, _c_vp]),
     "gbf_adjust_phi_f64": (ctypes.c_int, [_c_i32, _c_i32, _c_vp, _c_vp, _c_vp]),
     "gbf_face_geometry_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp]),
+    "gbf_cell_faces_work_ints": (ctypes.c_int64, [_c_i32, _c_i32, _c_i32]),
+    "gbf_cell_faces_device": (ctypes.c_int, [_c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp,
+                                             _c_vp, _c_vp, _c_vp, _c_vp, _c_vp]),
     "gbf_cell_faces": (ctypes.c_int, [_c_i32, _c_i32, _c_i32, _c_vp, _c_vp, _c_vp, _c_vp]),
     "gbf_cell_geometry_f64": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp,
                                              _c_vp, _c_vp, _c_vp, _c_vp]),

@@ -97,6 +97,154 @@ __global__ void __launch_bounds__(kBlock)
   st3(areas, f, a);
 }
 
+// ---- cell -> face lists ------------------------------------------------------
+// The order of the lists is the reference's visiting order: the owned faces
+// ascending, then the neighboured ones (as ~face) ascending.  Five launches:
+// counts, sums of 1024 counts, offsets, a fill in the order of arrival, and a
+// ranking that puts every entry in its place.  An entry's rank is found by
+// reading its cell's entries, one thread an entry: n loads of a line or two for
+// a cell of n faces, so a cell with more than kRankMax faces is left to the
+// host pass (status[1]).  64x48x40 hexahedra: 21 us, against 1360 us for the
+// host pass and 750 us for its 32-bit copies of owner and neighbour.
+constexpr unsigned int kRankMax = 4096;
+constexpr int kScanCells = 1024;
+
+// Faces whose cells lie outside [0, n_cells) are left out everywhere and the
+// lowest is recorded in status[0] (0xffffffff: none).
+__device__ __forceinline__ bool good_cell(int c, int n_cells) {
+  return (unsigned int)c < (unsigned int)n_cells;
+}
+
+__global__ void __launch_bounds__(kBlock)
+    list_count_kernel(int n_cells, int n_faces, int n_internal, const int64_t* __restrict__ owner,
+                      const int64_t* __restrict__ neighbour, int32_t* __restrict__ own32,
+                      int32_t* __restrict__ nei32, int32_t* __restrict__ count,
+                      uint32_t* __restrict__ status) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= n_faces) return;
+  const int o = (int)owner[f];
+  own32[f] = o;
+  bool good = good_cell(o, n_cells);
+  if (good) atomicAdd(count + o, 1);
+  if (f < n_internal) {
+    const int m = (int)neighbour[f];
+    nei32[f] = m;
+    if (good_cell(m, n_cells))
+      atomicAdd(count + m, 1);
+    else
+      good = false;
+  }
+  if (!good) atomicMin(status, (uint32_t)f);
+}
+
+__device__ __forceinline__ int block_sum_int(int v, int* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int t = 0;
+#pragma unroll
+  for (int w = 0; w < kBlock / 32; ++w) t += sh[w];
+  return t;
+}
+
+__global__ void __launch_bounds__(kBlock)
+    list_sums_kernel(int n_cells, const int32_t* __restrict__ count, int32_t* __restrict__ sums,
+                     uint32_t* __restrict__ status) {
+  __shared__ int sh[kBlock / 32];
+  int v = 0, most = 0;
+  for (int k = 0; k < kScanCells / kBlock; ++k) {
+    const long long c = (long long)blockIdx.x * kScanCells + k * kBlock + threadIdx.x;
+    const int n = c < n_cells ? count[c] : 0;
+    v += n;
+    most = max(most, n);
+  }
+  v = block_sum_int(v, sh);
+  if (threadIdx.x == 0) sums[blockIdx.x] = v;
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0) atomicMin(status + 1, ~(uint32_t)most);
+}
+
+// cell_ptr, and in place of the counts the position of each cell's first entry.
+__global__ void __launch_bounds__(kBlock)
+    list_offsets_kernel(int n_cells, int32_t* __restrict__ count, const int32_t* __restrict__ sums,
+                        int32_t* __restrict__ cell_ptr) {
+  __shared__ int sh[kBlock / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int before = 0;
+  for (int i = threadIdx.x; i < blockIdx.x; i += kBlock) before += sums[i];
+  before = block_sum_int(before, sh);
+  constexpr int K = kScanCells / kBlock;
+  const long long c0 = (long long)blockIdx.x * kScanCells + K * threadIdx.x;
+  int n[K], t = 0;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    n[k] = c0 + k < n_cells ? count[c0 + k] : 0;
+    t += n[k];
+  }
+  int scan = t;  // inclusive over the warp
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, scan, o);
+    if (lane >= o) scan += up;
+  }
+  __syncthreads();  // sh: still read by the sum above
+  if (lane == 31) sh[wid] = scan;
+  __syncthreads();
+  int at = before + scan - t;
+  for (int w = 0; w < wid; ++w) at += sh[w];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    if (c0 + k < n_cells) {
+      cell_ptr[c0 + k] = at;
+      count[c0 + k] = at;
+      at += n[k];
+      if (c0 + k == n_cells - 1) cell_ptr[n_cells] = at;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kBlock)
+    list_fill_kernel(int n_cells, int n_faces, int n_internal, const int32_t* __restrict__ own32,
+                     const int32_t* __restrict__ nei32, int32_t* __restrict__ at,
+                     int32_t* __restrict__ entries) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= n_faces) return;
+  const int o = own32[f];
+  if (good_cell(o, n_cells)) entries[atomicAdd(at + o, 1)] = f;
+  if (f < n_internal) {
+    const int m = nei32[f];
+    if (good_cell(m, n_cells)) entries[atomicAdd(at + m, 1)] = ~f;
+  }
+}
+
+// Owned faces before neighboured ones, each ascending, as unsigned keys.
+__device__ __forceinline__ uint32_t entry_key(int e) {
+  return e >= 0 ? (uint32_t)e : ~(uint32_t)e | 0x80000000u;
+}
+
+__global__ void __launch_bounds__(kBlock)
+    list_rank_kernel(int n_cells, int n_faces, int n_internal, const int32_t* __restrict__ own32,
+                     const int32_t* __restrict__ nei32, const int32_t* __restrict__ cell_ptr,
+                     const int32_t* __restrict__ entries, const uint32_t* __restrict__ status,
+                     int32_t* __restrict__ cell_faces) {
+  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  if (f >= n_faces || ~__ldg(status + 1) > kRankMax) return;
+#pragma unroll
+  for (int side = 0; side < 2; ++side) {
+    if (side == 1 && f >= n_internal) break;
+    const int c = side == 0 ? own32[f] : nei32[f];
+    if (!good_cell(c, n_cells)) continue;
+    const int e = side == 0 ? f : ~f;
+    const uint32_t key = entry_key(e);
+    const int q0 = __ldg(cell_ptr + c), q1 = __ldg(cell_ptr + c + 1);
+    int rank = 0;
+    for (int q = q0; q < q1; ++q) rank += entry_key(__ldg(entries + q)) < key;
+    cell_faces[q0 + rank] = e;
+  }
+}
+
 // Vertex k of face f as seen from a cell: reversed order on the cell's
 // neighbour-side faces (so that the face normal points out of the cell).
 __device__ __forceinline__ int face_vertex(const int32_t* __restrict__ face_pts, int b, int nv,
@@ -231,6 +379,39 @@ extern "C" int gbf_face_geometry_f64(int32_t n_faces, const int32_t* face_ptr,
               "face_geometry: NULL pointer");
   face_geometry_kernel<<<(n_faces + kBlock - 1) / kBlock, kBlock, 0, as_stream(stream)>>>(
       n_faces, face_ptr, face_pts, points, face_centres, face_areas);
+  GBF_CHECK_LAUNCH();
+  return GBF_OK;
+}
+
+extern "C" int64_t gbf_cell_faces_work_ints(int32_t n_cells, int32_t n_faces, int32_t n_internal) {
+  return (int64_t)n_cells + (n_cells + kScanCells - 1) / kScanCells + n_faces + n_internal;
+}
+
+extern "C" int gbf_cell_faces_device(int32_t n_cells, int32_t n_faces, int32_t n_internal,
+                                     const int64_t* owner, const int64_t* neighbour,
+                                     int32_t* owner32, int32_t* neighbour32, int32_t* cell_ptr,
+                                     int32_t* cell_faces, int32_t* work, uint32_t* status,
+                                     void* stream) {
+  GBF_REQUIRE(n_cells >= 1 && n_faces >= 1 && n_internal >= 0 && n_internal <= n_faces &&
+                  (int64_t)n_faces + n_internal <= INT32_MAX,
+              "cell_faces_device: bad counts");
+  GBF_REQUIRE(owner && owner32 && cell_ptr && cell_faces && work && status &&
+                  (n_internal == 0 || (neighbour && neighbour32)),
+              "cell_faces_device: NULL pointer");
+  cudaStream_t s = as_stream(stream);
+  const int nb = (int)(((int64_t)n_cells + kScanCells - 1) / kScanCells);
+  const int fb = (int)(((int64_t)n_faces + kBlock - 1) / kBlock);
+  int32_t *count = work, *sums = work + n_cells, *entries = sums + nb;
+  GBF_CHECK_CUDA(cudaMemsetAsync(count, 0, sizeof(int32_t) * (size_t)n_cells, s));
+  GBF_CHECK_CUDA(cudaMemsetAsync(status, 0xff, 2 * sizeof(uint32_t), s));
+  list_count_kernel<<<fb, kBlock, 0, s>>>(n_cells, n_faces, n_internal, owner, neighbour, owner32,
+                                          neighbour32, count, status);
+  list_sums_kernel<<<nb, kBlock, 0, s>>>(n_cells, count, sums, status);
+  list_offsets_kernel<<<nb, kBlock, 0, s>>>(n_cells, count, sums, cell_ptr);
+  list_fill_kernel<<<fb, kBlock, 0, s>>>(n_cells, n_faces, n_internal, owner32, neighbour32, count,
+                                         entries);
+  list_rank_kernel<<<fb, kBlock, 0, s>>>(n_cells, n_faces, n_internal, owner32, neighbour32,
+                                         cell_ptr, entries, status, cell_faces);
   GBF_CHECK_LAUNCH();
   return GBF_OK;
 }

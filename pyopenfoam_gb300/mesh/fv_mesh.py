@@ -6,8 +6,9 @@ The reference computes the geometry in Python loops over faces and cells
 (``mesh/mesh_geometry.py:35-395``: hours at 128^3).  Here the same formulas
 run as libgbfoam kernels, one thread per face or cell
 (``gbf_face_geometry_f64``, ``gbf_cell_geometry_f64``,
-``gbf_face_interp_f64``); the cell -> face lists come from one host pass
-(``gbf_cell_faces``).  Geometry is lazy and cached like the reference's;
+``gbf_face_interp_f64``), and so are the cell -> face lists
+(``gbf_cell_faces_device``; a mesh that it does not take, with no faces or a
+cell of more than 4096, goes through the host pass ``gbf_cell_faces``).  Geometry is lazy and cached like the reference's;
 ``compute_geometry()`` computes everything at once.
 
 Conventions are the reference's: faces are lists of point indices (or a
@@ -188,23 +189,42 @@ class FvMesh(PolyMesh):
     # ------------------------------------------------------------------
     def _addr(self) -> dict[str, torch.Tensor]:
         if self._dev_addr is None:
-            dev = self._device
-            n, nf, ni = self._n_cells, self._n_faces, self._n_internal_faces
-            own32 = np.ascontiguousarray(self._own_h, np.int32)
-            nei32 = np.ascontiguousarray(self._nei_h, np.int32)
-            cptr = np.empty(n + 1, np.int32)
-            cfaces = np.empty(max(nf + ni, 1), np.int32)
-            _lib.check(_lib.lib().gbf_cell_faces(n, nf, ni, own32.ctypes.data,
-                                                 nei32.ctypes.data, cptr.ctypes.data,
-                                                 cfaces.ctypes.data), "gbf_cell_faces")
-            to = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
-            self._dev_addr = dict(face_ptr=to(self._face_ptr_h),
-                                  face_pts=to(self._face_pts_h if self._face_pts_h.size
-                                              else np.zeros(1, np.int32)),
-                                  cell_ptr=to(cptr), cell_faces=to(cfaces),
-                                  owner32=to(own32 if own32.size else np.zeros(1, np.int32)),
-                                  neighbour32=to(nei32 if nei32.size else np.zeros(1, np.int32)))
+            to = lambda a: torch.from_numpy(a).to(self._device)  # noqa: E731
+            face_ptr = to(self._face_ptr_h)
+            face_pts = to(self._face_pts_h if self._face_pts_h.size else np.zeros(1, np.int32))
+            lists = self._cell_faces_device() or self._cell_faces_host()
+            self._dev_addr = dict(zip(("owner32", "neighbour32", "cell_ptr", "cell_faces"), lists),
+                                  face_ptr=face_ptr, face_pts=face_pts)
         return self._dev_addr
+
+    def _cell_faces_device(self) -> tuple[torch.Tensor, ...] | None:
+        """owner32, neighbour32, cell_ptr and cell_faces made on the device; None where its
+        kernels do not take the mesh (the host pass then makes them, or refuses)."""
+        n, nf, ni = self._n_cells, self._n_faces, self._n_internal_faces
+        if n < 1 or nf < 1 or ni > nf or nf + ni >= 2**31 or n >= 2**31:
+            return None
+        lib = _lib.lib()
+        empty = lambda k: torch.empty(k, dtype=torch.int32, device=self._device)  # noqa: E731
+        own32, nei32, cptr, cfaces = empty(nf), empty(max(ni, 1)), empty(n + 1), empty(nf + ni)
+        work, status = empty(lib.gbf_cell_faces_work_ints(n, nf, ni)), empty(2)
+        _lib.check(lib.gbf_cell_faces_device(
+            n, nf, ni, self._owner.data_ptr(), self._neighbour.data_ptr(), own32.data_ptr(),
+            nei32.data_ptr(), cptr.data_ptr(), cfaces.data_ptr(), work.data_ptr(),
+            status.data_ptr(), _lib.stream_ptr(self._device)), "gbf_cell_faces_device")
+        bad, most = status.tolist()
+        return (own32, nei32, cptr, cfaces) if bad == -1 and ~most <= 4096 else None
+
+    def _cell_faces_host(self) -> tuple[torch.Tensor, ...]:
+        n, nf, ni = self._n_cells, self._n_faces, self._n_internal_faces
+        own32 = np.ascontiguousarray(self._own_h, np.int32)
+        nei32 = np.ascontiguousarray(self._nei_h, np.int32)
+        cptr = np.empty(n + 1, np.int32)
+        cfaces = np.empty(max(nf + ni, 1), np.int32)
+        _lib.check(_lib.lib().gbf_cell_faces(n, nf, ni, own32.ctypes.data, nei32.ctypes.data,
+                                             cptr.ctypes.data, cfaces.ctypes.data),
+                   "gbf_cell_faces")
+        return tuple(torch.from_numpy(a if a.size else np.zeros(1, np.int32)).to(self._device)
+                     for a in (own32, nei32, cptr, cfaces))
 
     def _compute_face_geometry(self) -> None:
         if "face_centres" in self._geo:
