@@ -19,6 +19,7 @@
 
 #include "amul.cuh"
 #include "barrier.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
@@ -95,6 +96,9 @@ __device__ __forceinline__ float ldv_rw(const float* p, unsigned long long ef) {
 // that every thread of a tile takes the same branch.
 template <bool COH>
 __device__ __forceinline__ int tile_status(const BState* st) {
+  // A launch per phase: a status changes only when every tile of its system
+  // has read it (the last tile's ticket).
+  if constexpr (!COH) return st->status;
   __shared__ int s_status;
   __syncthreads();
   if (threadIdx.x == 0) s_status = ldc<COH>(&st->status);
@@ -103,12 +107,15 @@ __device__ __forceinline__ int tile_status(const BState* st) {
 }
 
 // True in every thread of the tile that finished last among its system's
-// tiles (count = number of tiles of the system); resets the ticket.
+// tiles (count = number of tiles of the system); resets the ticket.  Only
+// thread 0 wrote what the last tile reads (the partial sums), so it alone
+// fences before it takes the ticket.
 __device__ __forceinline__ bool last_tile_of_system(unsigned int* ticket, int count) {
   __shared__ bool am_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) am_last = (atomicAdd(ticket, 1u) == (unsigned)(count - 1));
+  if (threadIdx.x == 0) {
+    __threadfence();
+    am_last = (atomicAdd(ticket, 1u) == (unsigned)(count - 1));
+  }
   __syncthreads();
   if (am_last) {
     __threadfence();
@@ -137,7 +144,7 @@ __global__ void __launch_bounds__(BS)
                     const double* __restrict__ diag64, const double* __restrict__ pd,
                     const double* __restrict__ b, const double* __restrict__ x, BVecs v,
                     gbf_solve_params P) {
-  __shared__ double sh[BS / 32];
+  __shared__ double sh[2 * BS / 32];
   const int tile = blockIdx.x;
   const int s = __ldg(T.tile_sys + tile);
   double rr = 0.0, rz = 0.0;
@@ -156,19 +163,19 @@ __global__ void __launch_bounds__(BS)
     rr = fma(rh, rh, rr);
     rz += (double)r * (double)z;
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two<BS>(rr, rz, sh);
   if (threadIdx.x == 0) {
-    v.partials[tile] = rr;
-    v.partials[T.n_tiles + tile] = rz;
+    v.partials[tile] = sums.a;
+    v.partials[T.n_tiles + tile] = sums.b;
   }
   const int t0 = __ldg(T.sys_tile0 + s), t1 = __ldg(T.sys_tile0 + s + 1);
   BState* st = v.st + s;
   if (last_tile_of_system(&st->ticket[0], t1 - t0)) {
-    const double trr = tile_sum<BS>(v.partials, t0, t1, sh);
-    const double trz = tile_sum<BS>(v.partials + T.n_tiles, t0, t1, sh);
+    const SumPair total =
+        reduce_partials_two<BS>(v.partials + t0, v.partials + T.n_tiles + t0, t1 - t0, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res0 = res;
       st->res = res;
       st->rmax = res;
@@ -180,6 +187,17 @@ __global__ void __launch_bounds__(BS)
     }
   }
 }
+
+// A tile of a phase is bound by latency: the loads of a few cells per thread,
+// the reduction over the tile, and the chain of the system's last tile (fence,
+// ticket, partial sums, scalars).  So the vector phases issue the loads of
+// kAhead cells of a thread together (two at a time in the Amul phase were
+// slower, 10.8 against 10.1 us), the two sums of a phase share one tree, and
+// what the last tile needs of the state is loaded at the start.  24 systems of
+// 16^3 to 48^3 cells: update phase 10.3 -> 8.0 us, whole solve (448 iterations)
+// 15.9 -> 14.4 ms.  Programmatic dependent launches gave nothing here (the
+// phases of one wave leave no room for the next kernel's blocks).
+constexpr int kAhead = 4;
 
 // ---- one tile of each phase of the iteration --------------------------------
 // Ap = A p (FP32), p.Ap; the system's last tile forms alpha (or breakdown).
@@ -197,6 +215,7 @@ __device__ __forceinline__ void bmp_ap_tile(const gbf_layout& L, const BTiles& T
   const int s = __ldg(T.tile_sys + tile);
   BState* st = v.st + s;
   if (tile_status<COH>(st) != GBF_RUNNING) return;
+  const double rz = ldc<COH>(&st->rz);  // for the last tile
   BDFAcc a;
   const int c_end = __ldg(T.tile_end + tile);
   if constexpr (TPC == 1) {
@@ -234,7 +253,7 @@ __device__ __forceinline__ void bmp_ap_tile(const gbf_layout& L, const BTiles& T
         st->status = GBF_BREAKDOWN;
         atomicSub(v.running, 1);
       } else {
-        st->alpha = ldc<COH>(&st->rz) / pAp;
+        st->alpha = div_rn(rz, pAp);
       }
     }
   }
@@ -248,17 +267,34 @@ __device__ __forceinline__ void bmp_update_cells(const BTiles& T, int tile,
                                                  double* __restrict__ x, const BVecs& v,
                                                  float alpha, BDFAcc& arr, BDFAcc& arz) {
   const unsigned long long ef = l2_evict_first();
-  for (int c = __ldg(T.tile_begin + tile) + threadIdx.x; c < __ldg(T.tile_end + tile); c += BS) {
-    if constexpr (FOLD) {
-      x[c] = ldc<COH>(x + c) + (double)fmaf(alpha, ldc<COH>(v.p + c), ldc<COH>(v.xlo + c));
-      v.xlo[c] = 0.0f;
+  const int end = __ldg(T.tile_end + tile);
+  for (int c0 = __ldg(T.tile_begin + tile) + threadIdx.x; c0 < end; c0 += kAhead * BS) {
+    float Ap[kAhead], r[kAhead], rD[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + u * BS;
+      if (c < end) {
+        Ap[u] = ldv_ro<COH>(v.Ap + c, ef);
+        r[u] = ldv_rw<COH>(v.r + c, ef);
+        rD[u] = ld_nc_hint(v.rD + c, ef);  // rD: written before this launch
+      }
     }
-    const float r = fmaf(-alpha, ldv_ro<COH>(v.Ap + c, ef), ldv_rw<COH>(v.r + c, ef));
-    const float z = ld_nc_hint(v.rD + c, ef) * r;  // rD: written before this launch
-    st_hint(v.r + c, r, ef);
-    v.z[c] = z;
-    arr.add_prod(r, r);
-    arz.add_prod(r, z);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + u * BS;
+      if (c < end) {
+        if constexpr (FOLD) {
+          x[c] = ldc<COH>(x + c) + (double)fmaf(alpha, ldc<COH>(v.p + c), ldc<COH>(v.xlo + c));
+          v.xlo[c] = 0.0f;
+        }
+        const float rc = fmaf(-alpha, Ap[u], r[u]);
+        const float z = rD[u] * rc;
+        st_hint(v.r + c, rc, ef);
+        v.z[c] = z;
+        arr.add_prod(rc, rc);
+        arz.add_prod(rc, z);
+      }
+    }
   }
 }
 
@@ -274,25 +310,28 @@ __device__ __forceinline__ void bmp_update_tile(const BTiles& T, int tile, doubl
   if (tile_status<COH>(st) != GBF_RUNNING) return;
   const float alpha = (float)ldc<COH>(&st->alpha);
   const bool fold = ldc<COH>(&st->fold_pending) != 0;
+  // what the last tile needs of the state, loaded before it has to wait for it
+  const double rz_old = ldc<COH>(&st->rz), rmax_old = ldc<COH>(&st->rmax);
+  const double target = ldc<COH>(&st->target);
+  const int inner = ldc<COH>(&st->inner) + 1;
   BDFAcc arr, arz;
   if (fold)
     bmp_update_cells<BS, true, COH>(T, tile, x, v, alpha, arr, arz);
   else
     bmp_update_cells<BS, false, COH>(T, tile, x, v, alpha, arr, arz);
-  const double rr = block_sum_df(arr, sh);
-  const double rz = block_sum_df(arz, sh);
+  const SumPair sums = block_sum_df_two<BS>(arr, arz, sh);
   if (threadIdx.x == 0) {
-    v.partials[tile] = rr;
-    v.partials[T.n_tiles + tile] = rz;
+    v.partials[tile] = sums.a;
+    v.partials[T.n_tiles + tile] = sums.b;
   }
   const int t0 = __ldg(T.sys_tile0 + s), t1 = __ldg(T.sys_tile0 + s + 1);
   if (last_tile_of_system(&st->ticket[2], t1 - t0)) {
-    const double trr = tile_sum<BS>(v.partials, t0, t1, sh);
-    const double trz = tile_sum<BS>(v.partials + T.n_tiles, t0, t1, sh);
+    const SumPair total =
+        reduce_partials_two<BS>(v.partials + t0, v.partials + T.n_tiles + t0, t1 - t0, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
-      const int inner = ldc<COH>(&st->inner) + 1;
       st->inner = inner;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res = res;
       st->x_deferred = fold ? 0 : 1;  // the p phase adds alpha p to x32
       if (fold) {
@@ -300,11 +339,11 @@ __device__ __forceinline__ void bmp_update_tile(const BTiles& T, int tile, doubl
         st->phase = 1;
         if (COH) v.ctl->fold = 1;
       } else {
-        st->beta = trz / ldc<COH>(&st->rz);
+        st->beta = div_rn(trz, rz_old);
         st->rz = trz;
-        const double rmax = fmax(ldc<COH>(&st->rmax), res);
+        const double rmax = fmax(rmax_old, res);
         st->rmax = rmax;
-        if (res < delta * rmax || res < ldc<COH>(&st->target) || inner >= P.max_iter)
+        if (res < delta * rmax || res < target || inner >= P.max_iter)
           st->fold_pending = 1;
       }
     }
@@ -342,18 +381,18 @@ __device__ __forceinline__ void bmp_true_tile(const gbf_layout& L, const BTiles&
     rr = fma(rh, rh, rr);
     rz += (double)r * (double)z;
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two<BS>(rr, rz, sh);
   if (threadIdx.x == 0) {
-    v.partials[tile] = rr;
-    v.partials[T.n_tiles + tile] = rz;
+    v.partials[tile] = sums.a;
+    v.partials[T.n_tiles + tile] = sums.b;
   }
   const int t0 = __ldg(T.sys_tile0 + s), t1 = __ldg(T.sys_tile0 + s + 1);
   if (last_tile_of_system(&st->ticket[3], t1 - t0)) {
-    const double trr = tile_sum<BS>(v.partials, t0, t1, sh);
-    const double trz = tile_sum<BS>(v.partials + T.n_tiles, t0, t1, sh);
+    const SumPair total =
+        reduce_partials_two<BS>(v.partials + t0, v.partials + T.n_tiles + t0, t1 - t0, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       const int inner = ldc<COH>(&st->inner);
       st->res = res;
       st->updates = ldc<COH>(&st->updates) + 1;
@@ -365,7 +404,7 @@ __device__ __forceinline__ void bmp_true_tile(const gbf_layout& L, const BTiles&
         st->status = GBF_MAX_ITER;
         atomicSub(v.running, 1);
       } else {
-        st->beta = trz / ldc<COH>(&st->rz);
+        st->beta = div_rn(trz, ldc<COH>(&st->rz));
         st->rz = trz;
         st->rmax = res;
       }
@@ -391,10 +430,26 @@ __device__ __forceinline__ void bmp_p_tile(const BTiles& T, int tile, const BVec
   const float beta = s_ab[0], alpha = s_ab[1];
   const bool xd = s_flags[1] != 0;
   const unsigned long long ef = l2_evict_first();
-  for (int c = __ldg(T.tile_begin + tile) + threadIdx.x; c < __ldg(T.tile_end + tile); c += BS) {
-    const float pc = ldc<COH>(v.p + c);
-    if (xd) st_hint(v.xlo + c, fmaf(alpha, pc, ldv_rw<COH>(v.xlo + c, ef)), ef);
-    v.p[c] = fmaf(beta, pc, ldv_ro<COH>(v.z + c, ef));
+  const int end = __ldg(T.tile_end + tile);
+  for (int c0 = __ldg(T.tile_begin + tile) + threadIdx.x; c0 < end; c0 += kAhead * BS) {
+    float p[kAhead], z[kAhead], xl[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + u * BS;
+      if (c < end) {
+        p[u] = ldc<COH>(v.p + c);
+        z[u] = ldv_ro<COH>(v.z + c, ef);
+        if (xd) xl[u] = ldv_rw<COH>(v.xlo + c, ef);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int c = c0 + u * BS;
+      if (c < end) {
+        if (xd) st_hint(v.xlo + c, fmaf(alpha, p[u], xl[u]), ef);
+        v.p[c] = fmaf(beta, p[u], z[u]);
+      }
+    }
   }
 }
 
@@ -417,10 +472,10 @@ __global__ void __launch_bounds__(BS)
 }
 
 template <int BS>
-__global__ void __launch_bounds__(BS)
+__global__ void __launch_bounds__(BS, 1536 / BS)
     bmp_update_kernel(BTiles T, double* __restrict__ x, BVecs v, double delta,
                       gbf_solve_params P) {
-  __shared__ double sh[BS / 32];
+  __shared__ double sh[2 * BS / 32];
   bmp_update_tile<BS, false>(T, blockIdx.x, x, v, delta, P, sh);
 }
 
@@ -429,7 +484,7 @@ __global__ void __launch_bounds__(BS)
     bmp_true_kernel(gbf_layout L, BTiles T, const double* __restrict__ coef64,
                     const double* __restrict__ diag64, const double* __restrict__ b,
                     const double* __restrict__ x, BVecs v, gbf_solve_params P) {
-  __shared__ double sh[BS / 32];
+  __shared__ double sh[2 * BS / 32];
   bmp_true_tile<BS, false>(L, T, blockIdx.x, coef64, diag64, b, x, v, P, sh);
 }
 
@@ -561,7 +616,7 @@ __global__ void __launch_bounds__(BS, 1536 / BS)
                           const double* __restrict__ b, double* __restrict__ x, BVecs v,
                           double delta, gbf_solve_params P) {
   extern __shared__ int pref[];  // [n_systems + 1]
-  __shared__ double sh[BS / 32];
+  __shared__ double sh[2 * BS / 32];
   const unsigned G = gridDim.x;
   GridBarrier* bar = &v.ctl->bar;
   // statuses were set by the init kernel (a separate launch); the barrier

@@ -242,31 +242,33 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
   return t;
 }
 
-// Both block_sum(a) and block_sum(b), for blocks of kBlock threads, valid in
-// thread 0: lanes 0-15 of a warp carry a, lanes 16-31 b, so each level of the
+// Both block_sum(a) and block_sum(b), for blocks of BS threads, valid in thread
+// 0: lanes 0-15 of a warp carry a, lanes 16-31 b, so each level of the
 // two trees is one addition (an FP64 instruction takes 64 clocks of its SM
 // quarter on GB300, and a kernel with one cell a thread spends more of them on
-// its sums than on its cells).  `sh` holds 2 * kBlock / 32.
+// its sums than on its cells).  `sh` holds 2 * BS / 32.
 struct SumPair {
   double a, b;
 };
+template <int BS = kBlock>
 __device__ __forceinline__ SumPair block_sum_two(double a, double b, double* sh) {
-  static_assert(kBlock == 256, "eight warps");
+  constexpr int NW = BS / 32;
+  static_assert(NW == 4 || NW == 8 || NW == 16, "the warps of a block fill half a warp at most");
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const bool low = lane < 16;
   double v = (low ? a : b) + __shfl_xor_sync(0xffffffffu, low ? b : a, 16);
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
   __syncthreads();  // sh may still be read by a previous call
-  if ((lane & 15) == 0) sh[(low ? 0 : 8) + wid] = v;
+  if ((lane & 15) == 0) sh[(low ? 0 : NW) + wid] = v;
   __syncthreads();
   SumPair s{0.0, 0.0};
   if (wid == 0) {
     // block_sum's tree over 32 entries first adds zeros: -0.0 becomes +0.0
-    v = (lane & 15) < 8 ? sh[(low ? 0 : 8) + (lane & 7)] : 0.0;
+    v = (lane & 15) < NW ? sh[(low ? 0 : NW) + (lane & 15)] : 0.0;
     if (__double_as_longlong(v) == (long long)0x8000000000000000ULL) v = 0.0;
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
+    for (int o = NW / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o, 16);
     s.b = __shfl_sync(0xffffffffu, v, 16);
     s.a = v;
   }
@@ -319,10 +321,10 @@ __device__ __forceinline__ T reduce_partials(const T* partials, int n, T* sh) {
 // reduce_partials of two rows of n partials, results in thread 0.  Four rows
 // at a time: with eight, the kernels that end in it take 64 registers instead
 // of 40 and the PBiCGStab solves were 4 % slower.
+template <int BS = kBlock>
 __device__ __forceinline__ SumPair reduce_partials_two(const double* pa, const double* pb, int n,
                                                        double* sh) {
-  constexpr int U = 4;
-  const int B = blockDim.x;
+  constexpr int U = 4, B = BS;
   const int lane = threadIdx.x & 31;
   double va = 0.0, vb = 0.0;
   for (int w0 = threadIdx.x - lane; w0 < n; w0 += U * B) {  // by warps
@@ -341,7 +343,7 @@ __device__ __forceinline__ SumPair reduce_partials_two(const double* pa, const d
       }
     }
   }
-  return block_sum_two(va, vb, sh);
+  return block_sum_two<BS>(va, vb, sh);
 }
 
 // 0.0 + p without a floating-point add: p itself, except that -0.0 becomes
@@ -428,6 +430,49 @@ __device__ __forceinline__ double block_sum_df(const DFAcc& a, double* sh) {
     if (lane == 0) t = (double)hi + (double)lo;
   }
   return t;
+}
+
+// Both block_sum_df(a) and block_sum_df(b), in thread 0: the halves of a warp
+// carry one each, as in block_sum_two, which halves the two dependent chains.
+// `sh` holds 2 * BS / 32 doubles.
+template <int BS = kBlock>
+__device__ __forceinline__ SumPair block_sum_df_two(const DFAcc& a, const DFAcc& b, double* sh) {
+  constexpr int NW = BS / 32;
+  static_assert(NW == 4 || NW == 8 || NW == 16, "the warps of a block fill half a warp at most");
+  float2* s2 = reinterpret_cast<float2*>(sh);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool low = lane < 16;
+  // lane 16 + j adds b of lane 16 + j to b of lane j: df_add is not symmetric
+  const float oh = __shfl_xor_sync(0xffffffffu, low ? b.hi : a.hi, 16);
+  const float ol = __shfl_xor_sync(0xffffffffu, low ? b.lo : a.lo, 16);
+  float hi = low ? a.hi : oh, lo = low ? a.lo : ol;
+  df_add(hi, lo, low ? oh : b.hi, low ? ol : b.lo);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    const float h = __shfl_down_sync(0xffffffffu, hi, o, 16);
+    const float l = __shfl_down_sync(0xffffffffu, lo, o, 16);
+    df_add(hi, lo, h, l);
+  }
+  __syncthreads();  // sh may still be read by a previous call
+  if ((lane & 15) == 0) s2[(low ? 0 : NW) + wid] = make_float2(hi, lo);
+  __syncthreads();
+  SumPair s{0.0, 0.0};
+  if (wid == 0) {
+    const float2 e =
+        (lane & 15) < NW ? s2[(low ? 0 : NW) + (lane & 15)] : make_float2(0.0f, 0.0f);
+    hi = __fadd_rn(e.x, 0.0f);  // block_sum_df's tree over 32 entries first adds zeros
+    lo = __fadd_rn(e.y, 0.0f);
+#pragma unroll
+    for (int o = NW / 2; o > 0; o >>= 1) {
+      const float h = __shfl_down_sync(0xffffffffu, hi, o, 16);
+      const float l = __shfl_down_sync(0xffffffffu, lo, o, 16);
+      df_add(hi, lo, h, l);
+    }
+    const double t = (double)hi + (double)lo;
+    s.b = __shfl_sync(0xffffffffu, t, 16);
+    s.a = t;
+  }
+  return s;
 }
 
 }  // namespace gbf
