@@ -35,6 +35,7 @@
 #include <string.h>
 
 #include "bulk.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kBlock)
       if (fabs(pAp) < 1e-30)
         st->status = GBF_BREAKDOWN;
       else
-        st->alpha = st->rz / pAp;
+        st->alpha = div_rn(st->rz, pAp);
     }
   }
 }
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(kTileCells, kStreamBlocksPerSM)
       else if (fabs(pAp) < 1e-30)
         st->status = GBF_BREAKDOWN;
       else
-        st->alpha = st->rz / pAp;
+        st->alpha = div_rn(st->rz, pAp);
     }
   }
 }
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   const float alpha = (float)v.st->alpha;
   const bool fold = v.st->fold_pending != 0;
@@ -279,26 +280,25 @@ __global__ void __launch_bounds__(kBlock)
     mp_update_cells<true>(n, x, v, alpha, arr, arz);
   else
     mp_update_cells<false>(n, x, v, alpha, arr, arz);
-  const double rr = block_sum_df(arr, sh);
-  const double rz = block_sum_df(arz, sh);
+  const SumPair sums = block_sum_df_two(arr, arz, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = rr;
-    v.partials[G + blockIdx.x] = rz;
+    v.partials[blockIdx.x] = sums.a;
+    v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[2])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trz = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
       MixedState* st = v.st;
       st->inner += 1;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res = res;
       st->x_deferred = fold ? 0 : 1;  // K_p adds alpha p to x32
       if (fold) {
         st->fold_pending = 0;
         st->phase = MP_TRUE_RESIDUAL;  // K_true replaces r and sets beta
       } else {
-        st->beta = trz / st->rz;
+        st->beta = div_rn(trz, st->rz);
         st->rz = trz;
         st->rmax = fmax(st->rmax, res);
         if (res < delta * st->rmax || res < st->target || st->inner >= P.max_iter)
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING || v.st->phase != MP_TRUE_RESIDUAL) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   double rr = 0.0, rz = 0.0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += G * blockDim.x) {
@@ -328,18 +328,17 @@ __global__ void __launch_bounds__(kBlock)
     rr = fma(rh, rh, rr);
     rz += dprod(r, z);
   }
-  rr = block_sum(rr, sh);
-  rz = block_sum(rz, sh);
+  const SumPair sums = block_sum_two(rr, rz, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = rr;
-    v.partials[G + blockIdx.x] = rz;
+    v.partials[blockIdx.x] = sums.a;
+    v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[3])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trz = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
       MixedState* st = v.st;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res = res;
       st->updates += 1;
       if (st->n_hist < hist_cap) hist[st->n_hist] = res;
@@ -352,7 +351,7 @@ __global__ void __launch_bounds__(kBlock)
       } else if (st->inner >= P.max_iter) {
         st->status = GBF_MAX_ITER;
       } else {
-        st->beta = trz / st->rz;
+        st->beta = div_rn(trz, st->rz);
         st->rz = trz;
         st->rmax = res;
       }

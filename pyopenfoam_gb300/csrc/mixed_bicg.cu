@@ -33,6 +33,7 @@
 
 #include "barrier.cuh"
 #include "bulk.cuh"
+#include "exact.cuh"
 
 namespace gbf {
 
@@ -143,21 +144,26 @@ __device__ __forceinline__ void mb_amul_cell(const MbVecs& v, int c, float yv, f
 }
 
 // Block sums and the last block's scalar step of the two Amul kernels.
-template <int PH>
+template <int PH, int BS = kBlock>
 __device__ __forceinline__ void mb_amul_finish(const MbVecs& v, const DFAcc& a0,
                                                const DFAcc& a1, double* sh) {
   const int G = gridDim.x;
-  const double s0 = block_sum_df(a0, sh);
-  double s1 = 0.0;
-  if constexpr (PH == 1) s1 = block_sum_df(a1, sh);
+  SumPair sums{0.0, 0.0};
+  if constexpr (PH == 1)
+    sums = block_sum_df_two<BS>(a0, a1, sh);
+  else
+    sums.a = block_sum_df(a0, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = s0;
-    if constexpr (PH == 1) v.partials[G + blockIdx.x] = s1;
+    v.partials[blockIdx.x] = sums.a;
+    if constexpr (PH == 1) v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[1 + PH])) {
-    const double t0 = reduce_partials(v.partials, G, sh);
-    double t1 = 0.0;
-    if constexpr (PH == 1) t1 = reduce_partials(v.partials + G, G, sh);
+    SumPair total{0.0, 0.0};
+    if constexpr (PH == 1)
+      total = reduce_partials_two<BS>(v.partials, v.partials + G, G, sh);
+    else
+      total.a = reduce_partials(v.partials, G, sh);
+    const double t0 = total.a, t1 = total.b;
     if (threadIdx.x == 0) {
       MbState* st = v.st;
       if (__ldcg(&st->fault)) {
@@ -166,13 +172,13 @@ __device__ __forceinline__ void mb_amul_finish(const MbVecs& v, const DFAcc& a0,
         if (fabs(t0) < 1e-30)
           st->status = GBF_BREAKDOWN;  // pbicgstab.py:168-171
         else
-          st->alpha = st->rho / t0;
+          st->alpha = div_rn(st->rho, t0);
       } else {
         if (fabs(t0) < 1e-30) {
           st->branch = 1;  // pbicgstab.py:196-208
         } else {
           st->branch = 0;
-          st->omega = t1 / t0;
+          st->omega = div_rn(t1, t0);
         }
       }
     }
@@ -186,7 +192,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const float* __restrict__ src = PH == 0 ? v.y : v.z;
   DFAcc a0, a1;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells;
@@ -212,7 +218,7 @@ __global__ void __launch_bounds__(kTileCells, kStreamBlocksPerSM)
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ HexRing<false> ring;
-  __shared__ double sh[kTileCells / 32];
+  __shared__ double sh[2 * kTileCells / 32];
   const float* __restrict__ src = PH == 0 ? v.y : v.z;
   DFAcc a0, a1;
   const bool ok = hex_stream_tiles_pre<float, false, false>(
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(kTileCells, kStreamBlocksPerSM)
     }
   }
   if (!ok && threadIdx.x == 0) atomicExch(&v.st->fault, 1);
-  mb_amul_finish<PH>(v, a0, a1, sh);
+  mb_amul_finish<PH, kTileCells>(v, a0, a1, sh);
 }
 
 // s = r - alpha v, z = s / d_M, x32 += alpha y.  Four cells per thread with
@@ -347,7 +353,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   const int branch = v.st->branch;
   const float omega = (float)v.st->omega;
@@ -357,19 +363,18 @@ __global__ void __launch_bounds__(kBlock)
     mb_r_cells<true>(n, x, v, branch, omega, arr, artr);
   else
     mb_r_cells<false>(n, x, v, branch, omega, arr, artr);
-  const double rr = block_sum_df(arr, sh);
-  const double rtr = block_sum_df(artr, sh);
+  const SumPair sums = block_sum_df_two(arr, artr, sh);
   if (threadIdx.x == 0) {
-    v.partials[blockIdx.x] = rr;
-    v.partials[G + blockIdx.x] = rtr;
+    v.partials[blockIdx.x] = sums.a;
+    v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[3])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trtr = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trtr = total.b;
     if (threadIdx.x == 0) {
       MbState* st = v.st;
       st->inner += 1;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res = res;
       if (branch == 0 && fabs(st->omega) < 1e-30) {
         st->status = GBF_BREAKDOWN;  // pbicgstab.py:227-229
@@ -377,8 +382,8 @@ __global__ void __launch_bounds__(kBlock)
         st->fold_pending = 0;
         st->phase = MB_TRUE_RESIDUAL;  // K_true replaces r and sets beta
       } else {
-        st->beta = branch == 0 ? (trtr / st->rho) * (st->alpha / st->omega)
-                               : (trtr / st->rho) * st->alpha;
+        st->beta = branch == 0 ? div_rn(trtr, st->rho) * div_rn(st->alpha, st->omega)
+                               : div_rn(trtr, st->rho) * st->alpha;
         st->rho = trtr;
         st->rmax = fmax(st->rmax, res);
         if (res < delta * st->rmax || res < st->target || st->inner >= P.max_iter)
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING || v.st->phase != MB_TRUE_RESIDUAL) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
   double rr = 0.0;
   DFAcc artr;
@@ -417,11 +422,11 @@ __global__ void __launch_bounds__(kBlock)
     v.partials[G + blockIdx.x] = rtr;
   }
   if (last_block_done(&v.st->ticket[4])) {
-    const double trr = reduce_partials(v.partials, G, sh);
-    const double trtr = reduce_partials(v.partials + G, G, sh);
+    const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
+    const double trr = total.a, trtr = total.b;
     if (threadIdx.x == 0) {
       MbState* st = v.st;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       st->res = res;
       st->updates += 1;
       if (st->n_hist < hist_cap) hist[st->n_hist] = res;
@@ -432,8 +437,8 @@ __global__ void __launch_bounds__(kBlock)
       } else if (st->inner >= P.max_iter) {
         st->status = GBF_MAX_ITER;
       } else {
-        st->beta = st->branch == 0 ? (trtr / st->rho) * (st->alpha / st->omega)
-                                   : (trtr / st->rho) * st->alpha;
+        st->beta = st->branch == 0 ? div_rn(trtr, st->rho) * div_rn(st->alpha, st->omega)
+                                   : div_rn(trtr, st->rho) * st->alpha;
         st->rho = trtr;
         st->rmax = res;
         if (fabs(trtr) < 1e-30) st->status = GBF_BREAKDOWN;
@@ -544,7 +549,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const float beta = (float)v.st->beta;
   const float omega = v.st->branch == 0 ? (float)v.st->omega : 1.0f;
   const float* __restrict__ po = parity ? v.p2 : v.p;
@@ -578,7 +583,7 @@ __global__ void __launch_bounds__(kBlock)
   pdl_wait();
   pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
-  __shared__ double sh[kBlock / 32];
+  __shared__ double sh[2 * kBlock / 32];
   const float alpha = (float)v.st->alpha;
   const float* __restrict__ vn = parity ? v.v : v.v2;  // this iteration's v
   const float* __restrict__ r = v.r;
