@@ -286,11 +286,14 @@ __global__ void __launch_bounds__(kBlock)
     v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[2])) {
+    // read before the sums are waited for
+    const double rz_old = v.st->rz, rmax_old = v.st->rmax, target = v.st->target;
+    const int inner = v.st->inner + 1;
     const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
     const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
       MixedState* st = v.st;
-      st->inner += 1;
+      st->inner = inner;
       const double res = sqrt_rn(trr);
       st->res = res;
       st->x_deferred = fold ? 0 : 1;  // K_p adds alpha p to x32
@@ -298,10 +301,11 @@ __global__ void __launch_bounds__(kBlock)
         st->fold_pending = 0;
         st->phase = MP_TRUE_RESIDUAL;  // K_true replaces r and sets beta
       } else {
-        st->beta = div_rn(trz, st->rz);
+        st->beta = div_rn(trz, rz_old);
         st->rz = trz;
-        st->rmax = fmax(st->rmax, res);
-        if (res < delta * st->rmax || res < st->target || st->inner >= P.max_iter)
+        const double rmax = fmax(rmax_old, res);
+        st->rmax = rmax;
+        if (res < delta * rmax || res < target || inner >= P.max_iter)
           st->fold_pending = 1;
       }
     }

@@ -369,24 +369,29 @@ __global__ void __launch_bounds__(kBlock)
     v.partials[G + blockIdx.x] = sums.b;
   }
   if (last_block_done(&v.st->ticket[3])) {
+    // read before the sums are waited for
+    const double rho = v.st->rho, alpha = v.st->alpha, om = v.st->omega;
+    const double rmax_old = v.st->rmax, target = v.st->target;
+    const int inner = v.st->inner + 1;
     const SumPair total = reduce_partials_two(v.partials, v.partials + G, G, sh);
     const double trr = total.a, trtr = total.b;
     if (threadIdx.x == 0) {
       MbState* st = v.st;
-      st->inner += 1;
+      st->inner = inner;
       const double res = sqrt_rn(trr);
       st->res = res;
-      if (branch == 0 && fabs(st->omega) < 1e-30) {
+      if (branch == 0 && fabs(om) < 1e-30) {
         st->status = GBF_BREAKDOWN;  // pbicgstab.py:227-229
       } else if (fold) {
         st->fold_pending = 0;
         st->phase = MB_TRUE_RESIDUAL;  // K_true replaces r and sets beta
       } else {
-        st->beta = branch == 0 ? div_rn(trtr, st->rho) * div_rn(st->alpha, st->omega)
-                               : div_rn(trtr, st->rho) * st->alpha;
+        st->beta = branch == 0 ? div_rn(trtr, rho) * div_rn(alpha, om)
+                               : div_rn(trtr, rho) * alpha;
         st->rho = trtr;
-        st->rmax = fmax(st->rmax, res);
-        if (res < delta * st->rmax || res < st->target || st->inner >= P.max_iter)
+        const double rmax = fmax(rmax_old, res);
+        st->rmax = rmax;
+        if (res < delta * rmax || res < target || inner >= P.max_iter)
           st->fold_pending = 1;
         else if (fabs(trtr) < 1e-30)
           st->status = GBF_BREAKDOWN;  // the next iteration's rho test

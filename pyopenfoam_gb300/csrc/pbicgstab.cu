@@ -18,9 +18,12 @@
 // The vector kernels are bound by the FP64 pipe (64 clocks of its SM quarter
 // an instruction, an IEEE division several), not by their bytes: the products
 // and the divisions by the DILU diagonal run on the integer pipe (exact.cuh,
-// the same bits) and the two sums of K_t and K_r share one tree.  Measured for
-// a whole solve with DILU, before and after: 128x120x100 84.1 -> 62.5 ms (656
-// iterations), 72x60x50 in no order 16.3 -> 13.3 ms (320 iterations).
+// the same bits) and the two sums of K_t and K_r share one tree.  Each kernel
+// is a programmatic dependent launch of the one before, which takes the launch
+// out of the chain of a small system's five kernels.  Measured for a whole
+// solve with DILU, before, after the arithmetic, and after the launches:
+// 128x120x100 84.1, 62.5, 58.4 ms (656 iterations), 72x60x50 in no order 16.3,
+// 13.3, 11.8 ms (320), 40x30x30 5.1, 4.5, 3.6 ms (177).
 #include <math.h>
 #include <string.h>
 
@@ -95,6 +98,8 @@ template <int KIND>
 __global__ void __launch_bounds__(kBlock)
     bicg_v_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
                   BicgVecs v) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -115,7 +120,7 @@ __global__ void __launch_bounds__(kBlock)
       if (fabs(rtv) < 1e-30)
         st->status = GBF_BREAKDOWN;  // pbicgstab.py:168-171
       else
-        st->alpha = st->rho / rtv;
+        st->alpha = div_rn(st->rho, rtv);
     }
   }
 }
@@ -124,6 +129,8 @@ template <bool PREC>
 __global__ void __launch_bounds__(kBlock)
     bicg_s_kernel(int n, const double* __restrict__ pd, double* __restrict__ x, BicgVecs v,
                   double* hist, gbf_solve_params P) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -142,7 +149,7 @@ __global__ void __launch_bounds__(kBlock)
     const double tss = reduce_partials(v.partials, G, sh);
     if (threadIdx.x == 0) {
       BicgState* st = v.st;
-      const double res = sqrt(tss);
+      const double res = sqrt_rn(tss);
       hist[st->n_hist] = res;
       st->n_hist += 1;
       st->res = res;
@@ -156,6 +163,8 @@ template <int KIND>
 __global__ void __launch_bounds__(kBlock)
     bicg_t_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
                   BicgVecs v, int standard_omega) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -183,7 +192,7 @@ __global__ void __launch_bounds__(kBlock)
         st->branch = 1;  // pbicgstab.py:196-208
       } else {
         st->branch = 0;
-        st->omega = ttz / ttt;
+        st->omega = div_rn(ttz, ttt);
       }
     }
   }
@@ -191,6 +200,8 @@ __global__ void __launch_bounds__(kBlock)
 
 __global__ void __launch_bounds__(kBlock)
     bicg_r_kernel(int n, double* __restrict__ x, BicgVecs v, double* hist, gbf_solve_params P) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -219,7 +230,7 @@ __global__ void __launch_bounds__(kBlock)
     const double trr = total.a, trtr = total.b;
     if (threadIdx.x == 0) {
       BicgState* st = v.st;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       hist[st->n_hist] = res;
       st->n_hist += 1;
       st->res = res;
@@ -231,10 +242,10 @@ __global__ void __launch_bounds__(kBlock)
           if (fabs(st->omega) < 1e-30) {
             st->status = GBF_BREAKDOWN;  // pbicgstab.py:227-229
           } else {
-            st->beta = (rho_new / st->rho) * (st->alpha / st->omega);
+            st->beta = div_rn(rho_new, st->rho) * div_rn(st->alpha, st->omega);
           }
         } else {
-          st->beta = (rho_new / st->rho) * st->alpha;
+          st->beta = div_rn(rho_new, st->rho) * st->alpha;
         }
         st->rho = rho_new;
         if (st->status == GBF_RUNNING) {
@@ -252,6 +263,8 @@ __global__ void __launch_bounds__(kBlock)
 template <bool PREC>
 __global__ void __launch_bounds__(kBlock)
     bicg_p_kernel(int n, const double* __restrict__ pd, BicgVecs v) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   const double beta = v.st->beta;
   const double omega = v.st->omega;
@@ -325,20 +338,20 @@ extern "C" int gbf_pbicgstab_solve_f64(const gbf_layout* L, const double* coef,
   while (hs.status == GBF_RUNNING && launched < P->max_iter) {
     for (int j = 0; j < chunk && launched < P->max_iter; ++j, ++launched) {
       const bool tb = timing_begin(kProbeBicgAmul, s);
-      GBF_LAYOUT_DISPATCH(*L, K, bicg_v_kernel<K><<<G, kBlock, 0, s>>>(*L, coef, diag, v));
+      GBF_LAYOUT_DISPATCH(*L, K, launch_pdl(bicg_v_kernel<K>, G, kBlock, s, *L, coef, diag, v));
       if (tb) timing_end(kProbeBicgAmul, s);
       if (pd)
-        bicg_s_kernel<true><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
+        launch_pdl(bicg_s_kernel<true>, G, kBlock, s, n, pd, x, v, hist, *P);
       else
-        bicg_s_kernel<false><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
+        launch_pdl(bicg_s_kernel<false>, G, kBlock, s, n, pd, x, v, hist, *P);
       GBF_LAYOUT_DISPATCH(*L, K,
-                          bicg_t_kernel<K><<<G, kBlock, 0, s>>>(*L, coef, diag, v,
+                          launch_pdl(bicg_t_kernel<K>, G, kBlock, s, *L, coef, diag, v,
                                                                 P->variant == 1));
-      bicg_r_kernel<<<G, kBlock, 0, s>>>(n, x, v, hist, *P);
+      launch_pdl(bicg_r_kernel, G, kBlock, s, n, x, v, hist, *P);
       if (pd)
-        bicg_p_kernel<true><<<G, kBlock, 0, s>>>(n, pd, v);
+        launch_pdl(bicg_p_kernel<true>, G, kBlock, s, n, pd, v);
       else
-        bicg_p_kernel<false><<<G, kBlock, 0, s>>>(n, pd, v);
+        launch_pdl(bicg_p_kernel<false>, G, kBlock, s, n, pd, v);
     }
     GBF_CHECK_LAUNCH();
     GBF_CHECK_CUDA(cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s));

@@ -23,8 +23,9 @@
 // instruction), so alpha p and the division run on the integer pipe
 // (exact.cuh, the same bits; not alpha Ap as well: the two pipes are then
 // about even) and r.r and r.z share one tree.  Whole solves with DIC, before
-// and after: 120x110x100 72.2 -> 60.4 ms, 170x160x150 249.5 -> 173.1 ms,
-// 90x80x70 in no order 47.7 -> 39.2 ms (732, 926 and 553 iterations).
+// and after: 120x110x100 72.2 -> 60.4 ms, 170x160x150 249.5 -> 173.1 ms (168.9
+// with programmatic dependent launches), 90x80x70 in no order 47.7 -> 39.2 ms
+// (732, 926 and 553 iterations).
 #include <math.h>
 #include <string.h>
 
@@ -102,6 +103,8 @@ template <int KIND>
 __global__ void __launch_bounds__(kBlock)
     pcg_ap_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
                   PcgVecs v) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -123,7 +126,7 @@ __global__ void __launch_bounds__(kBlock)
       if (fabs(pAp) < 1e-30)
         st->status = GBF_BREAKDOWN;  // pcg.py:153-156: x returned as is
       else
-        st->alpha = st->rz / pAp;
+        st->alpha = div_rn(st->rz, pAp);
     }
   }
 }
@@ -132,6 +135,8 @@ template <bool PREC>
 __global__ void __launch_bounds__(kBlock)
     pcg_update_kernel(int n, const double* __restrict__ pd, double* __restrict__ x, PcgVecs v,
                       double* hist, gbf_solve_params P) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   __shared__ double sh[2 * kBlock / 32];
   const int G = gridDim.x;
@@ -158,14 +163,14 @@ __global__ void __launch_bounds__(kBlock)
     if (threadIdx.x == 0) {
       PcgState* st = v.st;
       const int it = st->iter;
-      const double res = sqrt(trr);
+      const double res = sqrt_rn(trr);
       hist[it] = res;
       st->res = res;
       st->n_hist = it + 1;
       if (monitor_converged(res, st->res0, it, P)) {
         st->status = GBF_CONVERGED;
       } else {
-        st->beta = trz / st->rz;
+        st->beta = div_rn(trz, st->rz);
         st->rz = trz;
         st->iter = it + 1;
         if (it >= P.max_iter) st->status = GBF_MAX_ITER;
@@ -175,6 +180,8 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 __global__ void __launch_bounds__(kBlock) pcg_p_kernel(int n, PcgVecs v) {
+  pdl_wait();
+  pdl_launch_dependents();
   if (v.st->status != GBF_RUNNING) return;
   const double beta = v.st->beta;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
@@ -873,15 +880,15 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
     for (int j = 0; j < chunk && launched < P->max_iter; ++j, ++launched) {
       const bool tb = timing_begin(kProbePcgAp, s);
       if (layout_kind(*L) == kLayoutHex33)
-        pcg_ap_kernel<kLayoutHex33><<<G, kBlock, 0, s>>>(*L, coef, diag, v);
+        launch_pdl(pcg_ap_kernel<kLayoutHex33>, G, kBlock, s, *L, coef, diag, v);
       else
-        pcg_ap_kernel<kLayoutGeneric><<<G, kBlock, 0, s>>>(*L, coef, diag, v);
+        launch_pdl(pcg_ap_kernel<kLayoutGeneric>, G, kBlock, s, *L, coef, diag, v);
       if (tb) timing_end(kProbePcgAp, s);
       if (pd)
-        pcg_update_kernel<true><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
+        launch_pdl(pcg_update_kernel<true>, G, kBlock, s, n, pd, x, v, hist, *P);
       else
-        pcg_update_kernel<false><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
-      pcg_p_kernel<<<G, kBlock, 0, s>>>(n, v);
+        launch_pdl(pcg_update_kernel<false>, G, kBlock, s, n, pd, x, v, hist, *P);
+      launch_pdl(pcg_p_kernel, G, kBlock, s, n, v);
     }
     GBF_CHECK_LAUNCH();
     GBF_CHECK_CUDA(cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s));
@@ -1012,14 +1019,14 @@ extern "C" int gbf_pcg_solve_f64_noalloc(const gbf_layout* L, const double* coef
   while (hs.status == GBF_RUNNING && launched < P->max_iter) {
     for (int j = 0; j < chunk && launched < P->max_iter; ++j, ++launched) {
       if (hex)
-        pcg_ap_kernel<kLayoutHex33><<<G, kBlock, 0, s>>>(*L, coef, diag, v);
+        launch_pdl(pcg_ap_kernel<kLayoutHex33>, G, kBlock, s, *L, coef, diag, v);
       else
-        pcg_ap_kernel<kLayoutGeneric><<<G, kBlock, 0, s>>>(*L, coef, diag, v);
+        launch_pdl(pcg_ap_kernel<kLayoutGeneric>, G, kBlock, s, *L, coef, diag, v);
       if (pd)
-        pcg_update_kernel<true><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
+        launch_pdl(pcg_update_kernel<true>, G, kBlock, s, n, pd, x, v, hist, *P);
       else
-        pcg_update_kernel<false><<<G, kBlock, 0, s>>>(n, pd, x, v, hist, *P);
-      pcg_p_kernel<<<G, kBlock, 0, s>>>(n, v);
+        launch_pdl(pcg_update_kernel<false>, G, kBlock, s, n, pd, x, v, hist, *P);
+      launch_pdl(pcg_p_kernel, G, kBlock, s, n, v);
     }
     GBF_CHECK_LAUNCH();
     GBF_CHECK_CUDA(cudaMemcpyAsync(&hs, v.st, sizeof(hs), cudaMemcpyDeviceToHost, s));
