@@ -607,14 +607,52 @@ extern "C" int gbf_explicit_laplacian_grad_d_f64(const gbf_layout* L, int32_t n_
 //   [+ sum_bnd -phi_b]) / V.
 // ---------------------------------------------------------------------------
 namespace gbf {
+// diag and source in one pass over a cell's faces: one read of the face lists
+// and all the face values of both sums in flight together (2097152 hexahedra:
+// 105 us, against 63 + 56 us as two kernels).  Each sum is cell_face_sum's.
 __global__ void __launch_bounds__(kBlock)
-    pressure_source_kernel(gbf_layout L, const int32_t* __restrict__ bnd_ptr,
-                           const int32_t* __restrict__ bnd_face, const double* __restrict__ phi,
-                           const double* __restrict__ V, int has_bnd, double* __restrict__ src) {
+    pressure_cell_kernel(gbf_layout L, const double* __restrict__ lower,
+                         const double* __restrict__ upper, const int32_t* __restrict__ bnd_ptr,
+                         const int32_t* __restrict__ bnd_face, const double* __restrict__ phi,
+                         const double* __restrict__ V, int has_bnd, double* __restrict__ diag,
+                         double* __restrict__ src) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= L.n_cells) return;
-  double y = cell_face_sum(
-      L, c, [&](int f) { return -__ldg(phi + f); }, [&](int f) { return __ldg(phi + f); });
+  double d = 0.0, y = 0.0;
+  if (L.n_faces > 0) {
+    const CellSlots cs = cell_slots(L, c);
+    if (cs.wo <= 4 && cs.wn <= 4) {
+      int f[8];
+      double v[8], g[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
+        f[4 + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        v[k] = f[k] >= 0 ? -__ldg((k < 4 ? lower : upper) + f[k]) : 0.0;
+        g[k] = f[k] >= 0 ? __ldg(phi + f[k]) : 0.0;
+      }
+      double vo = 0.0, vn = 0.0, go = 0.0, gn = 0.0;
+      if (f[0] >= 0) vo = first_term(v[0]), go = first_term(-g[0]);
+      if (f[4] >= 0) vn = first_term(v[4]), gn = first_term(g[4]);
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        if (f[k] >= 0) vo = __dadd_rn(vo, v[k]), go = __dsub_rn(go, g[k]);
+        if (f[4 + k] >= 0) vn = __dadd_rn(vn, v[4 + k]), gn = __dadd_rn(gn, g[4 + k]);
+      }
+      d = __dadd_rn(vo, vn);
+      y = __dadd_rn(go, gn);
+    } else {
+      d = cell_face_sum(
+          L, c, [&](int f) { return -__ldg(lower + f); },
+          [&](int f) { return -__ldg(upper + f); });
+      y = cell_face_sum(
+          L, c, [&](int f) { return -__ldg(phi + f); }, [&](int f) { return __ldg(phi + f); });
+    }
+  }
+  diag[c] = d;
   if (has_bnd) {
     double sb = 0.0;
     for (int k = __ldg(bnd_ptr + c); k < __ldg(bnd_ptr + c + 1); ++k)
@@ -651,11 +689,8 @@ extern "C" int gbf_pressure_assemble_f64(const gbf_layout* L, int32_t n_faces_to
         nint, L->owner, L->neighbour, face_areas, delta, D, volumes, lower, upper);
     GBF_CHECK_LAUNCH();
   }
-  lap_diag_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(
-      *L, lower, upper, nullptr, nullptr, face_areas, delta, D, volumes, 0, diag);
-  GBF_CHECK_LAUNCH();
-  pressure_source_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(
-      *L, bnd_ptr, bnd_face, phiHbyA, volumes, has_bnd ? 1 : 0, source);
+  pressure_cell_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(
+      *L, lower, upper, bnd_ptr, bnd_face, phiHbyA, volumes, has_bnd ? 1 : 0, diag, source);
   GBF_CHECK_LAUNCH();
   return GBF_OK;
 }
