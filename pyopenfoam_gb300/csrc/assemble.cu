@@ -24,32 +24,21 @@ __device__ __forceinline__ double face_smag(const double* __restrict__ a) {
 // Face diffusivity: constant, per face, or linearly interpolated from cells
 // (LinearInterpolation.interpolate, interpolation.py:101-145:
 //  w*phi_P + (1 - w)*phi_N on internal faces, phi_P on boundary faces).
-// Mode 3 is the pressure equation's 1/A_p: the per-cell values are
-// 1 / max(|A_p|, 1e-30) (pressure_equation.py:103-104), then interpolated
-// like mode 2.
 struct DiffSpec {
-  int mode;            // 0 constant, 1 per face, 2 per cell, 3 per-cell 1/|A_p|
+  int mode;            // 0 constant, 1 per face, 2 per cell
   double value;        // mode 0
   const double* face;  // mode 1: [n_faces]
-  const double* cell;  // modes 2, 3: [n_cells]
-  const double* w;     // modes 2, 3: [n_faces] interpolation weights
+  const double* cell;  // mode 2: [n_cells]
+  const double* w;     // mode 2: [n_faces] interpolation weights
 };
-
-__device__ __forceinline__ double cell_D(const DiffSpec& D, int c) {
-  const double v = __ldg(D.cell + c);
-  if (D.mode != 3) return v;
-  return div_rn(1.0, clamp_abs_min(v));  // clamp(min) keeps NaN
-}
 
 __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q, bool internal) {
   if (D.mode == 0) return D.value;
   if (D.mode == 1) return __ldg(D.face + f);
-  const double dp = cell_D(D, p);
+  const double dp = __ldg(D.cell + p);
   if (!internal) return dp;
-  const double w = __ldg(D.w + f), v = __dsub_rn(1.0, w), dq = cell_D(D, q);
-  // mode 3 divides twice on the integer pipe; mode 2 leaves it room for the products
-  if (D.mode == 2) return __dadd_rn(mul_int(w, dp), mul_int(v, dq));
-  return __dadd_rn(__dmul_rn(w, dp), __dmul_rn(v, dq));
+  const double w = __ldg(D.w + f), v = __dsub_rn(1.0, w), dq = __ldg(D.cell + q);
+  return __dadd_rn(mul_int(w, dp), mul_int(v, dq));
 }
 
 // (0 + sum over the cell's owner-side faces) + (sum over its neighbour-side
@@ -607,6 +596,14 @@ extern "C" int gbf_explicit_laplacian_grad_d_f64(const gbf_layout* L, int32_t n_
 //   [+ sum_bnd -phi_b]) / V.
 // ---------------------------------------------------------------------------
 namespace gbf {
+// 1 / max(|A_p|, 1e-30) of every cell (pressure_equation.py:103-104; the clamp
+// keeps NaN), which the faces interpolate.
+__global__ void __launch_bounds__(kBlock)
+    inv_diag_kernel(int n, const double* __restrict__ A, double* __restrict__ inv) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < n) inv[c] = div_rn(1.0, clamp_abs_min(__ldg(A + c)));
+}
+
 // diag and source in one pass over a cell's faces: one read of the face lists
 // and all the face values of both sums in flight together (2097152 hexahedra:
 // 105 us, against 63 + 56 us as two kernels).  Each sum is cell_face_sum's.
@@ -679,12 +676,17 @@ extern "C" int gbf_pressure_assemble_f64(const gbf_layout* L, int32_t n_faces_to
               "pressure_assemble: NULL pointer");
   const bool has_bnd = n_faces_total > nint;
   GBF_REQUIRE(!has_bnd || (bnd_ptr && bnd_face), "pressure_assemble: NULL boundary lists");
-  const DiffSpec D = make_spec(3, 0.0, nullptr, A_p, face_weights);
+  // The inverse of A_p is formed once a cell, in diag until that is written,
+  // and not twice a face: the face kernel is bound by the integer pipe, where
+  // it divides (2097152 hexahedra: 151 us, now 11 + 126 us).
+  const DiffSpec D = make_spec(2, 0.0, nullptr, diag, face_weights);
   cudaStream_t s = as_stream(stream);
   if (nint > 0) {
     GBF_REQUIRE(lower && upper && face_areas && delta && face_weights && L->owner &&
                     L->neighbour,
                 "pressure_assemble: NULL pointer");
+    inv_diag_kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(n, A_p, diag);
+    GBF_CHECK_LAUNCH();
     lap_face_kernel<<<(nint + kBlock - 1) / kBlock, kBlock, 0, s>>>(
         nint, L->owner, L->neighbour, face_areas, delta, D, volumes, lower, upper);
     GBF_CHECK_LAUNCH();
