@@ -24,12 +24,8 @@ __device__ __forceinline__ double inv_abs_clamped(double a) {
   return div_rn(1.0, max_abs_tiny(a));
 }
 
-// w*a + (1 - w)*b with each operation rounded.
-__device__ __forceinline__ double lerp_w(double w, double a, double b) {
-  return __dadd_rn(__dmul_rn(w, a), __dmul_rn(__dsub_rn(1.0, w), b));
-}
-
-// The same with both products on the integer pipe.
+// w*a + (1 - w)*b with each operation rounded, both products on the integer
+// pipe.
 __device__ __forceinline__ double lerp_int(double w, double v, double a, double b) {
   return __dadd_rn(mul_int(w, a), mul_int(v, b));  // v = 1 - w
 }

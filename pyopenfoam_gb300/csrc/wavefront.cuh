@@ -104,10 +104,6 @@ __device__ __forceinline__ void st_flow(double* p, double v) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
-__device__ __forceinline__ void st_flow_raw(double* p, long long bits) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(bits) : "memory");
-}
-
 __device__ __forceinline__ bool flow_empty(double v) {
   return __double_as_longlong(v) == kFlowEmpty;
 }
