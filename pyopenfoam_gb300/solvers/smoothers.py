@@ -59,7 +59,7 @@ class _GsSchedule:
         self.ptr_h = np.ascontiguousarray(ptr[: nl.value + 1])
         self.ptr = torch.from_numpy(self.ptr_h.copy()).to(topo.device)
         self.cells = torch.from_numpy(cells).to(topo.device)
-        self.blocks = block_order(cells[:n], topo.device)
+        self.blocks = block_order(self.cells[:n], topo.device)
 
 
 def _gs_schedule(matrix: LduMatrix, reverse: bool) -> _GsSchedule:
