@@ -191,13 +191,15 @@ __global__ void __launch_bounds__(BS)
 // A tile of a phase is bound by latency: the loads of a few cells per thread,
 // the reduction over the tile, and the chain of the system's last tile (fence,
 // ticket, partial sums, scalars).  So the vector phases issue the loads of
-// kAhead cells of a thread together (two at a time in the Amul phase were
+// four cells of a thread together (two at a time in the Amul phase were
 // slower, 10.8 against 10.1 us), the two sums of a phase share one tree, and
 // what the last tile needs of the state is loaded at the start.  24 systems of
 // 16^3 to 48^3 cells: update phase 10.3 -> 8.0 us, whole solve (448 iterations)
 // 15.9 -> 14.4 ms.  Programmatic dependent launches gave nothing here (the
 // phases of one wave leave no room for the next kernel's blocks).
-constexpr int kAhead = 4;
+// The persistent form keeps one cell: it has 40 registers for every phase.
+template <bool COH>
+constexpr int kAheadOf = COH ? 1 : 4;
 
 // ---- one tile of each phase of the iteration --------------------------------
 // Ap = A p (FP32), p.Ap; the system's last tile forms alpha (or breakdown).
@@ -215,7 +217,7 @@ __device__ __forceinline__ void bmp_ap_tile(const gbf_layout& L, const BTiles& T
   const int s = __ldg(T.tile_sys + tile);
   BState* st = v.st + s;
   if (tile_status<COH>(st) != GBF_RUNNING) return;
-  const double rz = ldc<COH>(&st->rz);  // for the last tile
+  const double rz_early = COH ? 0.0 : st->rz;  // for the last tile
   BDFAcc a;
   const int c_end = __ldg(T.tile_end + tile);
   if constexpr (TPC == 1) {
@@ -253,7 +255,7 @@ __device__ __forceinline__ void bmp_ap_tile(const gbf_layout& L, const BTiles& T
         st->status = GBF_BREAKDOWN;
         atomicSub(v.running, 1);
       } else {
-        st->alpha = div_rn(rz, pAp);
+        st->alpha = div_rn(COH ? ldc<COH>(&st->rz) : rz_early, pAp);
       }
     }
   }
@@ -267,6 +269,7 @@ __device__ __forceinline__ void bmp_update_cells(const BTiles& T, int tile,
                                                  double* __restrict__ x, const BVecs& v,
                                                  float alpha, BDFAcc& arr, BDFAcc& arz) {
   const unsigned long long ef = l2_evict_first();
+  constexpr int kAhead = kAheadOf<COH>;
   const int end = __ldg(T.tile_end + tile);
   for (int c0 = __ldg(T.tile_begin + tile) + threadIdx.x; c0 < end; c0 += kAhead * BS) {
     float Ap[kAhead], r[kAhead], rD[kAhead];
@@ -311,9 +314,16 @@ __device__ __forceinline__ void bmp_update_tile(const BTiles& T, int tile, doubl
   const float alpha = (float)ldc<COH>(&st->alpha);
   const bool fold = ldc<COH>(&st->fold_pending) != 0;
   // what the last tile needs of the state, loaded before it has to wait for it
-  const double rz_old = ldc<COH>(&st->rz), rmax_old = ldc<COH>(&st->rmax);
-  const double target = ldc<COH>(&st->target);
-  const int inner = ldc<COH>(&st->inner) + 1;
+  // (the persistent form, at its 40 registers, reads it at the end)
+  double rz_old, rmax_old, target;
+  int inner;
+  auto load_state = [&] {
+    rz_old = ldc<COH>(&st->rz);
+    rmax_old = ldc<COH>(&st->rmax);
+    target = ldc<COH>(&st->target);
+    inner = ldc<COH>(&st->inner) + 1;
+  };
+  if constexpr (!COH) load_state();
   BDFAcc arr, arz;
   if (fold)
     bmp_update_cells<BS, true, COH>(T, tile, x, v, alpha, arr, arz);
@@ -330,6 +340,7 @@ __device__ __forceinline__ void bmp_update_tile(const BTiles& T, int tile, doubl
         reduce_partials_two<BS>(v.partials + t0, v.partials + T.n_tiles + t0, t1 - t0, sh);
     const double trr = total.a, trz = total.b;
     if (threadIdx.x == 0) {
+      if constexpr (COH) load_state();
       st->inner = inner;
       const double res = sqrt_rn(trr);
       st->res = res;
@@ -430,6 +441,7 @@ __device__ __forceinline__ void bmp_p_tile(const BTiles& T, int tile, const BVec
   const float beta = s_ab[0], alpha = s_ab[1];
   const bool xd = s_flags[1] != 0;
   const unsigned long long ef = l2_evict_first();
+  constexpr int kAhead = kAheadOf<COH>;
   const int end = __ldg(T.tile_end + tile);
   for (int c0 = __ldg(T.tile_begin + tile) + threadIdx.x; c0 < end; c0 += kAhead * BS) {
     float p[kAhead], z[kAhead], xl[kAhead];
