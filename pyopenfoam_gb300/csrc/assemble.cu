@@ -47,40 +47,51 @@ __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q,
 // started at +0.0 is never -0.0, so adding it to 0.0 is the identity.  Up to
 // four slots a side (hex and most polyhedral cells) have every face index and
 // every face value of the cell in flight at once.
+//
+// M is the number of slots a side: an addition that no cell of the warp needs
+// holds the FP64 pipe all the same, so slices of three (hex cells) have a body
+// of their own; the widths are the slice's, so a warp takes one of them (983040
+// hexahedra: lap_diag_kernel 25.7 -> 22.8 us, div_diag_kernel 18.3 -> 16.7 us;
+// pressure_cell_kernel at 2097152, 105 -> 81 us).
+template <int M, typename O, typename N>
+__device__ __forceinline__ double few_face_sum(const gbf_layout& L, const CellSlots& cs, O&& own,
+                                               N&& nei) {
+  double so = 0.0, sn = 0.0, v[2 * M];
+  int f[2 * M];
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
+    f[M + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
+  }
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    v[k] = f[k] >= 0 ? own(f[k]) : 0.0;
+    v[M + k] = f[M + k] >= 0 ? nei(f[M + k]) : 0.0;
+  }
+  if (f[0] >= 0) so = first_term(v[0]);
+  if (f[M] >= 0) sn = first_term(v[M]);
+#pragma unroll
+  for (int k = 1; k < M; ++k) {
+    if (f[k] >= 0) so = __dadd_rn(so, v[k]);
+    if (f[M + k] >= 0) sn = __dadd_rn(sn, v[M + k]);
+  }
+  return __dadd_rn(so, sn);
+}
+
 template <typename O, typename N>
 __device__ __forceinline__ double cell_face_sum(const gbf_layout& L, int c, O&& own, N&& nei) {
-  double so = 0.0, sn = 0.0;
   if (L.n_faces == 0) return 0.0;
   const CellSlots cs = cell_slots(L, c);
-  if (cs.wo <= 4 && cs.wn <= 4) {
-    int f[8];
-    double v[8];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
-      f[4 + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = f[k] >= 0 ? own(f[k]) : 0.0;
-      v[4 + k] = f[4 + k] >= 0 ? nei(f[4 + k]) : 0.0;
-    }
-    if (f[0] >= 0) so = first_term(v[0]);
-    if (f[4] >= 0) sn = first_term(v[4]);
-#pragma unroll
-    for (int k = 1; k < 4; ++k) {
-      if (f[k] >= 0) so = __dadd_rn(so, v[k]);
-      if (f[4 + k] >= 0) sn = __dadd_rn(sn, v[4 + k]);
-    }
-  } else {
-    for (int k = 0; k < cs.wo; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * k);
-      if (f >= 0) so = __dadd_rn(so, own(f));
-    }
-    for (int k = 0; k < cs.wn; ++k) {
-      const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
-      if (f >= 0) sn = __dadd_rn(sn, nei(f));
-    }
+  if (cs.wo <= 3 && cs.wn <= 3) return few_face_sum<3>(L, cs, own, nei);
+  if (cs.wo <= 4 && cs.wn <= 4) return few_face_sum<4>(L, cs, own, nei);
+  double so = 0.0, sn = 0.0;
+  for (int k = 0; k < cs.wo; ++k) {
+    const int f = __ldg(L.slot_face + cs.base + 32 * k);
+    if (f >= 0) so = __dadd_rn(so, own(f));
+  }
+  for (int k = 0; k < cs.wn; ++k) {
+    const int f = __ldg(L.slot_face + cs.base + 32 * (cs.wo + k));
+    if (f >= 0) sn = __dadd_rn(sn, nei(f));
   }
   return __dadd_rn(so, sn);
 }
@@ -604,9 +615,39 @@ __global__ void __launch_bounds__(kBlock)
   if (c < n) inv[c] = div_rn(1.0, clamp_abs_min(__ldg(A + c)));
 }
 
+// The sums of pressure_cell_kernel for at most M slots a side (few_face_sum).
+template <int M>
+__device__ __forceinline__ void few_pressure_sums(const gbf_layout& L, const CellSlots& cs,
+                                                  const double* __restrict__ lower,
+                                                  const double* __restrict__ upper,
+                                                  const double* __restrict__ phi, double& d,
+                                                  double& y) {
+  int f[2 * M];
+  double v[2 * M], g[2 * M], vo = 0.0, vn = 0.0, go = 0.0, gn = 0.0;
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
+    f[M + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
+  }
+#pragma unroll
+  for (int k = 0; k < 2 * M; ++k) {
+    v[k] = f[k] >= 0 ? -__ldg((k < M ? lower : upper) + f[k]) : 0.0;
+    g[k] = f[k] >= 0 ? __ldg(phi + f[k]) : 0.0;
+  }
+  if (f[0] >= 0) vo = first_term(v[0]), go = first_term(-g[0]);
+  if (f[M] >= 0) vn = first_term(v[M]), gn = first_term(g[M]);
+#pragma unroll
+  for (int k = 1; k < M; ++k) {
+    if (f[k] >= 0) vo = __dadd_rn(vo, v[k]), go = __dsub_rn(go, g[k]);
+    if (f[M + k] >= 0) vn = __dadd_rn(vn, v[M + k]), gn = __dadd_rn(gn, g[M + k]);
+  }
+  d = __dadd_rn(vo, vn);
+  y = __dadd_rn(go, gn);
+}
+
 // diag and source in one pass over a cell's faces: one read of the face lists
 // and all the face values of both sums in flight together (2097152 hexahedra:
-// 105 us, against 63 + 56 us as two kernels).  Each sum is cell_face_sum's.
+// 81 us, against 63 + 56 us as two kernels).  Each sum is cell_face_sum's.
 __global__ void __launch_bounds__(kBlock)
     pressure_cell_kernel(gbf_layout L, const double* __restrict__ lower,
                          const double* __restrict__ upper, const int32_t* __restrict__ bnd_ptr,
@@ -618,29 +659,10 @@ __global__ void __launch_bounds__(kBlock)
   double d = 0.0, y = 0.0;
   if (L.n_faces > 0) {
     const CellSlots cs = cell_slots(L, c);
-    if (cs.wo <= 4 && cs.wn <= 4) {
-      int f[8];
-      double v[8], g[8];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        f[k] = k < cs.wo ? __ldg(L.slot_face + cs.base + 32 * k) : -1;
-        f[4 + k] = k < cs.wn ? __ldg(L.slot_face + cs.base + 32 * (cs.wo + k)) : -1;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        v[k] = f[k] >= 0 ? -__ldg((k < 4 ? lower : upper) + f[k]) : 0.0;
-        g[k] = f[k] >= 0 ? __ldg(phi + f[k]) : 0.0;
-      }
-      double vo = 0.0, vn = 0.0, go = 0.0, gn = 0.0;
-      if (f[0] >= 0) vo = first_term(v[0]), go = first_term(-g[0]);
-      if (f[4] >= 0) vn = first_term(v[4]), gn = first_term(g[4]);
-#pragma unroll
-      for (int k = 1; k < 4; ++k) {
-        if (f[k] >= 0) vo = __dadd_rn(vo, v[k]), go = __dsub_rn(go, g[k]);
-        if (f[4 + k] >= 0) vn = __dadd_rn(vn, v[4 + k]), gn = __dadd_rn(gn, g[4 + k]);
-      }
-      d = __dadd_rn(vo, vn);
-      y = __dadd_rn(go, gn);
+    if (cs.wo <= 3 && cs.wn <= 3) {
+      few_pressure_sums<3>(L, cs, lower, upper, phi, d, y);
+    } else if (cs.wo <= 4 && cs.wn <= 4) {
+      few_pressure_sums<4>(L, cs, lower, upper, phi, d, y);
     } else {
       d = cell_face_sum(
           L, c, [&](int f) { return -__ldg(lower + f); },
