@@ -50,7 +50,7 @@ __device__ __forceinline__ double face_D(const DiffSpec& D, int f, int p, int q,
 //
 // M is the number of slots a side: an addition that no cell of the warp needs
 // holds the FP64 pipe all the same, so slices of three (hex cells) have a body
-// of their own; the widths are the slice's, so a warp takes one of them (983040
+// of their own; the widths are the slice's, so a warp takes one of them (497664
 // hexahedra: lap_diag_kernel 25.7 -> 22.8 us, div_diag_kernel 18.3 -> 16.7 us;
 // pressure_cell_kernel at 2097152, 105 -> 81 us).
 template <int M, typename O, typename N>
