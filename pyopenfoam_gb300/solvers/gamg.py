@@ -300,10 +300,11 @@ class GAMGSolver(LinearSolverBase):
 
     def _cycle(self, matrix: LduMatrix, levels, aggs) -> dict:
         """One V-cycle plus the residual norm on static buffers, captured
-        once into a CUDA graph per hierarchy (the cycle is a few dozen
-        small launches, so replaying the graph removes the per-launch host
-        cost); eager launches if capture is off or fails."""
-        key = ("gamg_cycle", id(levels))
+        once into a CUDA graph per hierarchy and sweep counts (the cycle is a
+        few dozen small launches, so replaying the graph removes the
+        per-launch host cost); eager launches if capture is off or fails."""
+        key = ("gamg_cycle", id(levels), self._n_pre_smooth, self._n_post_smooth,
+               self._use_graph)
         hit = matrix._csr_cache.get(key)
         if hit is not None:
             return hit
