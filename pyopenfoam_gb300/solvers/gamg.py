@@ -246,23 +246,23 @@ class GAMGSolver(LinearSolverBase):
                 r: torch.Tensor) -> None:
         _lib.check(_lib.lib().gbf_jacobi_f64(
             m.topology().layout_ref, m.packed().data_ptr(), m.diag.data_ptr(), b.data_ptr(), 1.0,
-            int(n_it), x.data_ptr(), r.data_ptr(), _lib.stream_ptr(m.device)), "gbf_jacobi_f64")
+            n_it, x.data_ptr(), r.data_ptr(), _lib.stream_ptr(m.device)), "gbf_jacobi_f64")
 
-    def _v_cycle(self, levels, aggs, i: int, x: torch.Tensor, b: torch.Tensor, tail) -> None:
+    def _v_cycle(self, levels, aggs, i: int, x: torch.Tensor, b: torch.Tensor, tail,
+                 sweeps) -> None:
         m = levels[i].matrix
         st = _lib.stream_ptr(m.device)
         L = _lib.lib()
-        first, desc = tail
+        (first, desc), (pre, post) = tail, sweeps
         if i == first:
-            _lib.check(L.gbf_gamg_tail_f64(desc, len(desc), self._n_pre_smooth,
-                                           self._n_post_smooth, 50, b.data_ptr(), x.data_ptr(),
-                                           st), "gbf_gamg_tail_f64")
+            _lib.check(L.gbf_gamg_tail_f64(desc, len(desc), pre, post, 50, b.data_ptr(),
+                                           x.data_ptr(), st), "gbf_gamg_tail_f64")
             return
         r = torch.empty_like(x)
         if i == len(levels) - 1:
             self._jacobi(m, x, b, 50, r)
             return
-        self._jacobi(m, x, b, self._n_pre_smooth, r)
+        self._jacobi(m, x, b, pre, r)
         residual(m, b, x, r)
         agg = aggs[i]
         rc = torch.empty(agg.n_coarse, device=m.device, dtype=torch.float64)
@@ -271,10 +271,10 @@ class GAMGSolver(LinearSolverBase):
                                                  agg.agg_cells.data_ptr(), r.data_ptr(),
                                                  rc.data_ptr(), ec.data_ptr(), st),
                    "gbf_gamg_restrict_start_f64")
-        self._v_cycle(levels, aggs, i + 1, ec, rc, tail)
+        self._v_cycle(levels, aggs, i + 1, ec, rc, tail, sweeps)
         _lib.check(L.gbf_gamg_prolong_add_f64(m.n_cells, agg.f2c32.data_ptr(), ec.data_ptr(),
                                               x.data_ptr(), st), "gbf_gamg_prolong_add_f64")
-        self._jacobi(m, x, b, self._n_post_smooth, r)
+        self._jacobi(m, x, b, post, r)
 
     def _solve(self, matrix: LduMatrix, source: torch.Tensor, x0: torch.Tensor,
                monitor: ResidualMonitor, max_iter: int) -> tuple[torch.Tensor, ConvergenceInfo]:
@@ -303,8 +303,10 @@ class GAMGSolver(LinearSolverBase):
         once into a CUDA graph per hierarchy and sweep counts (the cycle is a
         few dozen small launches, so replaying the graph removes the
         per-launch host cost); eager launches if capture is off or fails."""
-        key = ("gamg_cycle", id(levels), self._n_pre_smooth, self._n_post_smooth,
-               self._use_graph)
+        # as range() counts them: none below zero, no fractions; one level has none
+        sweeps = tuple(len(range(k)) if len(levels) > 1 else 0
+                       for k in (self._n_pre_smooth, self._n_post_smooth))
+        key = ("gamg_cycle", id(levels), sweeps, self._use_graph)
         hit = matrix._csr_cache.get(key)
         if hit is not None:
             return hit
@@ -320,7 +322,7 @@ class GAMGSolver(LinearSolverBase):
         tail = self._tail(levels, aggs)
 
         def body():
-            self._v_cycle(levels, aggs, 0, buf["x"], buf["b"], tail)
+            self._v_cycle(levels, aggs, 0, buf["x"], buf["b"], tail, sweeps)
             _lib.check(L.gbf_residual_norm2_f64(
                 matrix.topology().layout_ref, matrix.packed().data_ptr(), matrix.diag.data_ptr(),
                 buf["b"].data_ptr(), buf["x"].data_ptr(), buf["r"].data_ptr(),

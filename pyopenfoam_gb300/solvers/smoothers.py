@@ -161,11 +161,12 @@ class JacobiSmoother:
         m = self._matrix
         x = _f64(m, x, "x").clone()
         b = _f64(m, b, "b")
-        if n_iterations > 0:
+        n_sweeps = len(range(n_iterations))  # none below zero, no fractions
+        if n_sweeps > 0:
             r = torch.empty_like(x)
             _lib.check(_lib.lib().gbf_jacobi_f64(
                 m.topology().layout_ref, m.packed().data_ptr(), m.diag.data_ptr(), b.data_ptr(),
-                float(self._omega), int(n_iterations), x.data_ptr(), r.data_ptr(),
+                float(self._omega), n_sweeps, x.data_ptr(), r.data_ptr(),
                 _lib.stream_ptr(m.device)), "gbf_jacobi_f64")
         return x
 
