@@ -766,16 +766,30 @@ static size_t pcg_base_bytes(int n) {
          align256(sizeof(PcgState));
 }
 
-// Sum words of pcg_resident_kernel on G blocks.
-static size_t resident_words(int G) {
-  return (size_t)G * 2 * kSlotSets * G;
+// Bytes of pcg_resident_kernel's sum words on G blocks.
+static size_t resident_bytes(long long G) {
+  return align256((size_t)G * 2 * kSlotSets * G * sizeof(TurnWord));
 }
 
+// What a solve of n cells can use: grows with n, so that a workspace for the
+// largest of several systems is one for each.  A system too large for the
+// resident kernel needs no sum words, but asks for no less than the largest
+// that is not.  Without a device there is no resident kernel.
 extern "C" size_t gbf_pcg_workspace_bytes(int32_t n) {
   if (n < 0) return 0;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    sms = 0;
+    cudaGetLastError();  // no device: not an error of this query
+  }
+  long long most = (long long)kResidentPerSM * sms;
+  if (most > kResidentMaxBlocks) most = kResidentMaxBlocks;
+  const size_t base = pcg_base_bytes(n);
   const long long G = ((long long)n + kBlock - 1) / kBlock;
-  return pcg_base_bytes(n) +
-         (G <= kResidentMaxBlocks ? align256(resident_words((int)G) * sizeof(TurnWord)) : 0);
+  if (G <= most) return base + resident_bytes(G);
+  const size_t largest = pcg_base_bytes((int)(most * kBlock)) + resident_bytes(most);
+  return base > largest ? base : largest;
 }
 
 extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const double* diag,
@@ -798,7 +812,9 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
     return GBF_OK;
   }
   GBF_REQUIRE(diag && b && x && hist && ws && (L->n_faces == 0 || coef), "pcg: NULL pointer");
-  GBF_REQUIRE(ws_bytes >= gbf_pcg_workspace_bytes(n), "pcg: workspace too small");
+  // the resident kernel's sum words are not required: without them the
+  // multi-cell kernel runs, with the same bits
+  GBF_REQUIRE(ws_bytes >= pcg_base_bytes(n), "pcg: workspace too small");
   cudaStream_t s = as_stream(stream);
 
   char* w = static_cast<char*>(ws);
@@ -817,8 +833,11 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
   // single launch (variant 2, or variant 0 on a launch-bound system)
   if (P->variant == 2 || (P->variant == 0 && n <= kPersistentMaxCells)) {
     const bool hex = layout_kind(*L) == kLayoutHex33;
-    const bool resident = pd ? resident_fits<true>(*L, hex) : resident_fits<false>(*L, hex);
-    const int Gp = resident ? (n + kBlock - 1) / kBlock
+    const int Gr = (n + kBlock - 1) / kBlock;
+    const bool resident =
+        (pd ? resident_fits<true>(*L, hex) : resident_fits<false>(*L, hex)) &&
+        ws_bytes >= pcg_base_bytes(n) + resident_bytes(Gr);
+    const int Gp = resident ? Gr
                    : hex ? (pd ? persistent_grid<kLayoutHex33, true>(n)
                              : persistent_grid<kLayoutHex33, false>(n))
                        : (pd ? persistent_grid<kLayoutGeneric, true>(n)
@@ -830,7 +849,7 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
         TurnWord* zw = reinterpret_cast<TurnWord*>(w);
         TurnWord* sw = reinterpret_cast<TurnWord*>(w + pcg_base_bytes(n));
         GBF_CHECK_CUDA(cudaMemsetAsync(zw, 0, 2 * sizeof(TurnWord) * (size_t)n, s));
-        GBF_CHECK_CUDA(cudaMemsetAsync(sw, 0, resident_words(Gp) * sizeof(TurnWord), s));
+        GBF_CHECK_CUDA(cudaMemsetAsync(sw, 0, resident_bytes(Gp), s));
         gbf_layout Lc = *L;
         gbf_solve_params Pc = *P;
         void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&pd, (void*)&b, &x, &zw, &sw,
