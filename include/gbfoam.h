@@ -373,7 +373,8 @@ typedef struct gbf_solve_result {
  * gbf_pcg_solve_f64 needs no more than four vectors of n_cells doubles, each
  * rounded up to 256 bytes, and 65,792 bytes; the rest is room for the
  * cell-per-thread kernel of small hex systems, without which a slower kernel
- * gives the same bits.                                                      */
+ * gives the same bits.  So it does in a workspace aligned to 8 bytes and not
+ * to 16.                                                                    */
 size_t gbf_pcg_workspace_bytes(int32_t n_cells);
 /* PCGSolver._solve, solvers/pcg.py:97-187.  x holds x0 on entry and the
  * solution on return.  precond_d = factorised DIC/DILU diagonal (z = r/d) or

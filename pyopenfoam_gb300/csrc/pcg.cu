@@ -834,9 +834,12 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
   if (P->variant == 2 || (P->variant == 0 && n <= kPersistentMaxCells)) {
     const bool hex = layout_kind(*L) == kLayoutHex33;
     const int Gr = (n + kBlock - 1) / kBlock;
+    // its words are written and read whole, 16 bytes at a 16-byte boundary;
+    // everything else in the workspace takes 8
     const bool resident =
         (pd ? resident_fits<true>(*L, hex) : resident_fits<false>(*L, hex)) &&
-        ws_bytes >= pcg_base_bytes(n) + resident_bytes(Gr);
+        ws_bytes >= pcg_base_bytes(n) + resident_bytes(Gr) &&
+        reinterpret_cast<uintptr_t>(ws) % alignof(TurnWord) == 0;
     const int Gp = resident ? Gr
                    : hex ? (pd ? persistent_grid<kLayoutHex33, true>(n)
                              : persistent_grid<kLayoutHex33, false>(n))

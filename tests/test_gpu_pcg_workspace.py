@@ -82,3 +82,13 @@ def test_the_query_grows_with_the_system():
     assert all(a <= b for a, b in zip(got, got[1:]))
     assert all(least_bytes(n) <= g <= max(least_bytes(n), query(last)) for n, g in zip(ns, got)
                if n > last)
+
+
+@pytest.mark.parametrize("dims", [(6, 5, 4), (32, 32, 32)])
+def test_a_workspace_aligned_to_eight_bytes(dims):
+    m, b = system(dims)
+    pd, n = DICPreconditioner(m).precond_diag, m.n_cells
+    nbytes = _lib.lib().gbf_pcg_workspace_bytes(n)
+    want, its, _ = solve(m, b, pd, nbytes)
+    got, it, _ = solve(m, b, pd, nbytes, offset=8)
+    assert it == its and all(torch.equal(g, w) for g, w in zip(got, want))
