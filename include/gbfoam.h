@@ -114,6 +114,11 @@ int gbf_selftest_wavefront_fault(int32_t* result_h);
  * the fault word (1 expected), result_h[1] = 1 if the output is all NaN.
  * No GPU fault is involved.                                                */
 int gbf_selftest_flow_fault(int32_t* result_h);
+/* Self-test of the cell-per-thread PCG kernel's failure path: a block that
+ * waits for a value that nothing publishes (1000-poll limit).  result_h[0] =
+ * the fault word (1 expected), result_h[1] = 1 if x is unchanged.  No GPU
+ * fault is involved.                                                        */
+int gbf_selftest_pcg_resident_fault(int32_t* result_h);
 /* Kernel timing probes (no reference counterpart; used by the benchmark to
  * time the dominant kernel inside a solve).  While enabled, the solvers
  * bracket the launches of their Amul kernels with CUDA events on the

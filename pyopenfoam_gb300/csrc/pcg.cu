@@ -27,6 +27,7 @@
 // with programmatic dependent launches), 90x80x70 in no order 47.7 -> 39.2 ms
 // (732, 926 and 553 iterations).
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include "amul.cuh"
@@ -440,9 +441,9 @@ __device__ __forceinline__ double block_sum_one(double v, double* sh, int count)
 }
 
 // One unsuccessful round of polls; false when the wait has run out.
-__device__ __forceinline__ bool poll_again(long long& polls, int* fault) {
+__device__ __forceinline__ bool poll_again(long long& polls, long long most, int* fault) {
   ++polls;
-  if (polls > kBarrierPolls || ((polls & 63) == 0 && *(volatile int*)fault != 0)) {
+  if (polls > most || ((polls & 63) == 0 && *(volatile int*)fault != 0)) {
     atomicExch(fault, 1);
     return false;
   }
@@ -493,7 +494,8 @@ __global__ void __launch_bounds__(kBlock, kResidentPerSM)
     pcg_resident_kernel(gbf_layout L, const double* __restrict__ coef,
                         const double* __restrict__ diag, const double* __restrict__ pd,
                         const double* __restrict__ b, double* __restrict__ x_io, TurnWord* z_all,
-                        TurnWord* slots, PcgState* st, double* hist, gbf_solve_params P) {
+                        TurnWord* slots, PcgState* st, double* hist, gbf_solve_params P,
+                        long long max_polls) {
   __shared__ double sh[16], ps[kBlock], bc[2], sent[2];
   const int G = gridDim.x, n = L.n_cells, tid = threadIdx.x, blk = blockIdx.x;
   const int c0 = blk * kBlock, c = c0 + tid;
@@ -570,7 +572,7 @@ __global__ void __launch_bounds__(kBlock, kResidentPerSM)
       if (want1) w1 = ld_word(p1);
       if (want0 && w0.turn == number) v0 = w0.v, want0 = false;
       if (want1 && w1.turn == number) v1 = w1.v, want1 = false;
-      if ((want0 || want1) && !poll_again(polls, fault)) {
+      if ((want0 || want1) && !poll_again(polls, max_polls, fault)) {
         ok = false;
         return;
       }
@@ -855,8 +857,9 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
         GBF_CHECK_CUDA(cudaMemsetAsync(sw, 0, resident_bytes(Gp), s));
         gbf_layout Lc = *L;
         gbf_solve_params Pc = *P;
+        long long polls = kBarrierPolls;
         void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&pd, (void*)&b, &x, &zw, &sw,
-                        &v.st, &hist, &Pc};
+                        &v.st, &hist, &Pc, &polls};
         e = cudaLaunchCooperativeKernel(pd ? (const void*)pcg_resident_kernel<true>
                                            : (const void*)pcg_resident_kernel<false>,
                                         dim3(Gp), dim3(kBlock), args, 0, s);
@@ -921,6 +924,63 @@ extern "C" int gbf_pcg_solve_f64(const gbf_layout* L, const double* coef, const 
   R->final_residual = hs.res;
   R->initial_residual = hs.res0;
   R->launches = 1 + 3 * launched;
+  return GBF_OK;
+}
+
+// Self-test of the cell-per-thread kernel's bounded waits, without a GPU fault:
+// one block of a system of two, whose cell 255 has a face to cell 256 of the
+// block that is not launched.  Nothing publishes that cell's z, so the wait
+// runs out after 1000 polls (about a millisecond), the fault word is set, the
+// block returns and x stays as it was.  result_h[0] = the fault word (1
+// expected), [1] = 1 if x is unchanged.  Every index stays inside the buffers.
+extern "C" int gbf_selftest_pcg_resident_fault(int32_t* result_h) {
+  GBF_REQUIRE(result_h, "selftest: NULL pointer");
+  int dev = 0, coop = 0;
+  GBF_CHECK_CUDA(cudaGetDevice(&dev));
+  GBF_CHECK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  GBF_REQUIRE(coop, "selftest: the device has no cooperative launch");
+  constexpr int n = 2 * kBlock, slices = n / 32;
+  struct Buf {
+    TurnWord z[2 * n], sums[2 * kSlotSets];
+    double coef[192 * slices], diag[n], b[n], x[n], hist[2];
+    int32_t dm[12 * slices];
+    PcgState st;
+  };
+  Buf* h = static_cast<Buf*>(calloc(1, sizeof(Buf)));
+  GBF_REQUIRE(h, "selftest: out of memory");
+  for (int i = 0; i < n; ++i) h->diag[i] = 4.0, h->b[i] = h->x[i] = 1.0;
+  const int last = kBlock / 32 - 1;  // slice of cell 255: its first slot, lane 31 alone
+  h->dm[12 * last] = 1;
+  h->dm[12 * last + 1] = (int32_t)0x80000000u;
+  Buf* d = nullptr;
+  cudaError_t e = cudaMalloc(&d, sizeof(Buf));
+  if (e == cudaSuccess) e = cudaMemcpy(d, h, sizeof(Buf), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    gbf_layout L;
+    memset(&L, 0, sizeof(L));
+    L.n_cells = n;
+    L.slot_dm = d->dm;
+    gbf_solve_params P;
+    memset(&P, 0, sizeof(P));
+    P.max_iter = 1;
+    const double *coef = d->coef, *diag = d->diag, *pd = nullptr, *b = d->b;
+    double *x = d->x, *hist = d->hist;
+    TurnWord *z = d->z, *sums = d->sums;
+    PcgState* st = &d->st;
+    long long polls = 1000;
+    void* args[] = {&L, (void*)&coef, (void*)&diag, (void*)&pd, (void*)&b, &x, &z, &sums,
+                    &st, &hist, &P, &polls};
+    e = cudaLaunchCooperativeKernel((const void*)pcg_resident_kernel<false>, dim3(1),
+                                    dim3(kBlock), args, 0, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(Buf), cudaMemcpyDeviceToHost);
+  }
+  if (d) cudaFree(d);
+  int same = 1;
+  for (int i = 0; i < n; ++i) same &= h->x[i] == 1.0 ? 1 : 0;
+  result_h[0] = h->st.bar.fault;
+  result_h[1] = same;
+  free(h);
+  GBF_CHECK_CUDA(e);
   return GBF_OK;
 }
 
