@@ -46,12 +46,17 @@ class FlowLinks:
 @dataclass
 class BlockOrder:
     """Cells of a level schedule dealt to resident blocks: block b takes the
-    cells [b * per, (b + 1) * per), in level order at cells[ptr[b]:ptr[b + 1]]."""
+    cells [b * per, (b + 1) * per), in level order at cells[ptr[b]:ptr[b + 1]].
+    ``share``: chunks of 32 cells that a level has on its busiest block, in the
+    mean over the levels; ``pays``: whether the block walk is then the faster
+    one (see ``WALK_SHARE_MAX``)."""
 
     ptr: torch.Tensor
     cells: torch.Tensor
     n_blocks: int
     per: int
+    share: float = 0.0
+    pays: bool = True
 
 
 #: Cells a block of a block walk may keep in shared memory (8 bytes each; a
@@ -60,13 +65,33 @@ class BlockOrder:
 #: between neighbouring cells stay inside it.
 WALK_CELLS_MAX = 24576
 WALK_CELLS_MIN = 512
+#: Largest ``share`` with which the block walk runs.  A level moves on when its
+#: busiest block has done its cells, eight chunks of 32 at a time at best, and
+#: in many numberings a front lies on few blocks: the walk over the whole
+#: schedule deals it to all of them.  Time by blocks over time of the whole
+#: schedule, DIC and Gauss-Seidel: share 1.0 (67x59x53 in mesh order) 0.89 and
+#: 0.97, 2.4 (100^3) 0.92 and 1.00, 3.0 (128^3) 1.13 and 1.62, 8.4 (1000x1000
+#: shuffled in runs of 64) 1.42 and 3.3.  Blocks of WALK_CELLS_MIN cells, two
+#: chunks a warp, are the faster walk in every numbering measured (40^3
+#: renumbered, share 3.7, 0.92 and 0.72).
+WALK_SHARE_MAX = 2.5
+#: The same where slices have more than four slots a side: such cells take
+#: their values one by one or repeat their row, so that the shorter trips
+#: inside a block count for more.  Share 1.0 (64^3, 10 % renumbered) 0.74 and
+#: 0.50, 3.0 (100^3, 60 % renumbered) 0.72 and 0.74, 3.9 (67x59x53 shuffled in
+#: runs of 4096) 1.19 and 0.88, 8.5 (67x59x53 renumbered) 1.24 and 1.12, 71
+#: (128^3 renumbered) 2.3 and 2.5.
+WALK_SHARE_MAX_WIDE = 3.8
 
 
-def block_order(level_cells: torch.Tensor | np.ndarray,
-                device: torch.device) -> BlockOrder | None:
+def block_order(level_cells: torch.Tensor | np.ndarray, device: torch.device,
+                level_ptr: torch.Tensor | None = None,
+                max_width: int = 0) -> BlockOrder | None:
     """The block order of a schedule's cells (each cell once), or None when a
     block per SM cannot keep its share of them.  Made on the device: the host's
-    sort was 7 ms of a first solve of 10^6 cells."""
+    sort was 7 ms of a first solve of 10^6 cells.  ``level_ptr`` (device, where
+    each level begins) gives the order its ``share``, which ``max_width`` (slots
+    of the layout's widest slice) judges."""
     n = level_cells.shape[0]
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     per = max(WALK_CELLS_MIN, -(-n // sms))
@@ -75,11 +100,23 @@ def block_order(level_cells: torch.Tensor | np.ndarray,
     n_blocks = -(-n // per)
     cells = torch.as_tensor(level_cells, device=device)
     block = torch.div(cells, per, rounding_mode="floor").to(torch.int16)
-    cells = cells[torch.sort(block, stable=True).indices]
+    by_block = torch.sort(block, stable=True).indices
+    cells, share = cells[by_block], 0.0
+    if level_ptr is not None:
+        n_levels = level_ptr.shape[0] - 1
+        level = torch.repeat_interleave(torch.arange(n_levels, device=device), level_ptr.diff(),
+                                        output_size=n)
+        key, count = torch.unique_consecutive(block[by_block].long() * n_levels + level[by_block],
+                                              return_counts=True)
+        most = torch.zeros(n_levels, dtype=torch.int64, device=device)
+        most.scatter_reduce_(0, key % n_levels, (count + 31) // 32, "amax")
+        share = int(most.sum()) / n_levels
     ptr = np.minimum(np.arange(n_blocks + 1, dtype=np.int64) * per, n).astype(np.int32)
     # the copy from pageable memory waits for the stream, so the order is
     # complete for whichever stream uses it
-    return BlockOrder(torch.from_numpy(ptr).to(device), cells, n_blocks, per)
+    limit = WALK_SHARE_MAX if max_width <= 8 else WALK_SHARE_MAX_WIDE
+    return BlockOrder(torch.from_numpy(ptr).to(device), cells, n_blocks, per, share,
+                      per == WALK_CELLS_MIN or share <= limit)
 
 
 def _i32_host(t: torch.Tensor, n_cells: int, name: str) -> np.ndarray:
@@ -228,7 +265,9 @@ class Topology:
     def dic_blocks(self) -> BlockOrder | None:
         """``dic_schedule()``'s cells dealt to blocks (see ``block_order``)."""
         if not self._dic_blocks_made:
-            self._dic_blocks = block_order(self.dic_schedule().items[: self.n_cells], self.device)
+            sch = self.dic_schedule()
+            self._dic_blocks = block_order(sch.items[: self.n_cells], self.device,
+                                           sch.ptr[: sch.n_levels + 1], self.max_width)
             self._dic_blocks_made = True
         return self._dic_blocks
 

@@ -56,7 +56,7 @@ def factor_dic(topo, coef: torch.Tensor, diag: torch.Tensor, d: torch.Tensor, de
     L, st = _lib.lib(), _lib.stream_ptr(device)
     bar = None if form == "per_level" else _lib.wavefront_barrier(device)
     blocks = topo.dic_blocks() if form == "flow" else None
-    if blocks is not None:
+    if blocks is not None and blocks.pays:
         _lib.check(L.gbf_dic_build_block_f64(topo.layout_ref, coef.data_ptr(), diag.data_ptr(),
                                              blocks.cells.data_ptr(), blocks.ptr.data_ptr(),
                                              blocks.n_blocks, blocks.per, d.data_ptr(),

@@ -59,7 +59,7 @@ class _GsSchedule:
         self.ptr_h = np.ascontiguousarray(ptr[: nl.value + 1])
         self.ptr = torch.from_numpy(self.ptr_h.copy()).to(topo.device)
         self.cells = torch.from_numpy(cells).to(topo.device)
-        self.blocks = block_order(self.cells[:n], topo.device)
+        self.blocks = block_order(self.cells[:n], topo.device, self.ptr, topo.max_width)
 
 
 def _gs_schedule(matrix: LduMatrix, reverse: bool) -> _GsSchedule:
@@ -91,7 +91,7 @@ def gs_sweep(matrix: LduMatrix, x: torch.Tensor, b: torch.Tensor, reverse: bool 
     st = _lib.stream_ptr(matrix.device)
     if form == "flow":
         scratch = torch.empty(max(matrix.n_cells, 1), dtype=torch.float64, device=matrix.device)
-        if sch.blocks is not None:
+        if sch.blocks is not None and sch.blocks.pays:
             bl = sch.blocks
             _lib.check(_lib.lib().gbf_gauss_seidel_block_f64(
                 topo.layout_ref, coef.data_ptr(), matrix.diag.data_ptr(), b.data_ptr(),
