@@ -338,29 +338,28 @@ __device__ __forceinline__ double row_result(double ax, double bc, double dc, do
 // bound by the FP64 pipe (16 operations a cell; 262144 cells: residual 8.9 us,
 // sweep 11.3 us, against 8.9 + 1.8 us of a sweep as two kernels with a
 // division per cell in the second).
-template <bool SWEEP>
+template <int KIND, bool SWEEP>
 __global__ void __launch_bounds__(kBlock)
-    hex_rows_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
-                    const double* __restrict__ b, double omega, const double* __restrict__ x,
-                    double* __restrict__ out) {
+    cell_rows_kernel(gbf_layout L, const double* __restrict__ coef, const double* __restrict__ diag,
+                     const double* __restrict__ b, double omega, const double* __restrict__ x,
+                     double* __restrict__ out) {
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < L.n_cells; c += gridDim.x * blockDim.x) {
     const double xc = __ldg(x + c);
-    const double ax =
-        cell_amul_k<kLayoutHex33, double, double, false>(L, coef, diag, x, c, xc);
+    const double ax = cell_amul_k<KIND, double, double, false>(L, coef, diag, x, c, xc);
     out[c] = row_result<SWEEP>(ax, __ldg(b + c), SWEEP ? __ldg(diag + c) : 1.0, xc, omega);
   }
 }
 
-// The same on any other layout (coarse multigrid levels, random numberings): a
-// block per 32-cell slice.  A thread per cell walks its row of 10-25 slots
-// through a chain of loads (offset entry, column, x) and of FP64 operations,
-// each of which holds the warp's SM quarter for 64 clocks: 10 us a level
-// however small.  Here the block's warps take the slots in turn (products into
-// shared memory), so all of the slice's loads are in flight together, and then
-// one warp sums the owner side and another the neighbour side in slot order --
-// the products and the order of cell_amul, so its bits: 1148 cells 10.2 -> 3.6
-// us, 8094 cells 9.8 -> 3.8, 32768 cells 10.0 -> 6.6, 131072 cells 15.0 -> 12.8
-// us a sweep.
+// The same on a small layout of any other kind (coarse multigrid levels,
+// random numberings), a block per 32-cell slice.  A thread per cell walks its
+// row of 10-25 slots through a chain of loads (offset entry, column, x) and of
+// FP64 operations, each of which holds the warp's SM quarter for 64 clocks: 10
+// us a level however small.  Here the block's warps take the slots in turn
+// (products into shared memory), so all of the slice's loads are in flight
+// together, and then one warp sums the owner side and another the neighbour
+// side in slot order -- the products and the order of cell_amul, so its bits:
+// 1148 cells 10.2 -> 3.6 us, 8094 cells 9.8 -> 3.8, 32768 cells 10.0 -> 5.0 us a
+// sweep.
 // The two summing warps differ from block to block, so that the sums do not
 // all fall on the same quarter of an SM.
 constexpr int kRowSlots = 32;  // slots of a slice held at a time
@@ -425,22 +424,42 @@ __global__ void __launch_bounds__(32 * kRowWarps)
   }
 }
 
-// Slices that eight warps each keep resident at once (8 blocks on 152 SMs);
-// above, four warps a slice.
-constexpr int kRowFewSlices = 8 * 152;
+// Which of the kernels, by the slices an SM has.  Eight warps a slice while the
+// device holds them all at once (eight blocks an SM), four above.  From
+// kRowThreadSlices on the device is full with a thread per cell too, and the
+// products need no trip through shared memory: residual of 91125 renumbered
+// cells (18.7 slices an SM) 8.9 us against 8.8, of 74088 (15.2) 6.8 against 8.6,
+// of 125000 11.4 against 9.9, of 2097152 166 against 123, of the first coarse
+// level of 200^3 332 against 200.  Not on slices so wide that a thread per cell
+// waits for the longest row of its warp: 250000 cells of a graph, slices of 20
+// slots in the mean and 155 at most, 31 us against 88; up to kRowThreadWidth the
+// two are within a fifth of each other (64^3 with 12 more neighbours a cell,
+// renumbered, widest slice 32, 40 against 49; 128^3 so, 34, 324 against 291).
+constexpr int kRowFewSlices = 8, kRowThreadSlices = 18;  // an SM
+constexpr int kRowThreadWidth = 40;
 
 template <bool SWEEP>
-static void launch_rows(const gbf_layout* L, const double* coef, const double* diag,
-                        const double* b, double omega, const double* x, double* out,
-                        cudaStream_t s) {
+static int launch_rows(const gbf_layout* L, const double* coef, const double* diag,
+                       const double* b, double omega, const double* x, double* out,
+                       cudaStream_t s) {
+  int32_t sms = 0;
+  const int rc = gbf_device_sm_count(&sms);
+  if (rc) return rc;
   if (layout_kind(*L) == kLayoutHex33) {
-    const int grid = wave_grid(hex_rows_kernel<SWEEP>, kBlock, L->n_cells);
-    hex_rows_kernel<SWEEP><<<grid, kBlock, 0, s>>>(*L, coef, diag, b, omega, x, out);
-  } else if (L->n_slices <= kRowFewSlices) {
+    const int grid = wave_grid(cell_rows_kernel<kLayoutHex33, SWEEP>, kBlock, L->n_cells);
+    cell_rows_kernel<kLayoutHex33, SWEEP>
+        <<<grid, kBlock, 0, s>>>(*L, coef, diag, b, omega, x, out);
+  } else if (L->n_slices > (int64_t)kRowThreadSlices * sms && L->max_width <= kRowThreadWidth) {
+    const int grid = wave_grid(cell_rows_kernel<kLayoutGeneric, SWEEP>, kBlock, L->n_cells);
+    cell_rows_kernel<kLayoutGeneric, SWEEP>
+        <<<grid, kBlock, 0, s>>>(*L, coef, diag, b, omega, x, out);
+  } else if (L->n_slices <= (int64_t)kRowFewSlices * sms) {
     slice_rows_kernel<SWEEP, 8><<<L->n_slices, 256, 0, s>>>(*L, coef, diag, b, omega, x, out);
   } else {
     slice_rows_kernel<SWEEP, 4><<<L->n_slices, 128, 0, s>>>(*L, coef, diag, b, omega, x, out);
   }
+  GBF_CHECK_LAUNCH();
+  return GBF_OK;
 }
 
 // x += (omega * s_c) * z with s_c = 1 / max(|diag_c|, 1e-30), or
@@ -672,9 +691,7 @@ extern "C" int gbf_residual_f64(const gbf_layout* L, const double* coef, const d
   if (L->n_cells == 0) return GBF_OK;
   GBF_REQUIRE(diag && b && x && r && (L->n_faces == 0 || coef), "residual: NULL pointer");
   cudaStream_t s = as_stream(stream);
-  launch_rows<false>(L, coef, diag, b, 1.0, x, r, s);
-  GBF_CHECK_LAUNCH();
-  return GBF_OK;
+  return launch_rows<false>(L, coef, diag, b, 1.0, x, r, s);
 }
 
 extern "C" int gbf_jacobi_f64(const gbf_layout* L, const double* coef, const double* diag,
@@ -689,12 +706,12 @@ extern "C" int gbf_jacobi_f64(const gbf_layout* L, const double* coef, const dou
   cudaStream_t s = as_stream(stream);
   double *from = x, *to = scratch;
   for (int k = 0; k < n_sweeps; ++k) {
-    launch_rows<true>(L, coef, diag, b, omega, from, to, s);
+    rc = launch_rows<true>(L, coef, diag, b, omega, from, to, s);
+    if (rc) return rc;
     double* t = from;
     from = to;
     to = t;
   }
-  GBF_CHECK_LAUNCH();
   if (from != x)  // an odd number of sweeps ends in the scratch
     GBF_CHECK_CUDA(cudaMemcpyAsync(x, from, sizeof(double) * (size_t)L->n_cells,
                                    cudaMemcpyDeviceToDevice, s));

@@ -13,7 +13,7 @@ from pyopenfoam_gb300.solvers import GAMGSolver, JacobiSmoother
 from pyopenfoam_gb300.solvers.smoothers import residual
 
 pytestmark = pytest.mark.gpu
-ROW_SLOTS, FEW_SLICES, TAIL_ROWS = 32, 8 * 152, 8192
+ROW_SLOTS, TAIL_ROWS = 32, 8192
 
 
 def matrix(n, own, nei, rng):
@@ -54,17 +54,27 @@ def sweep(m, b, x, omega):
 
 SYSTEMS = {"few_slices": lambda: renumbered((31, 29, 27)),
            "many_slices": lambda: renumbered((48, 40, 37)),
+           "cells": lambda: renumbered((60, 50, 41)),
+           "cells_2d": lambda: renumbered((330, 300, 1)),
            "one_slice": lambda: graph(30, 200),
-           "wide": lambda: graph(1003, 16000),
-           "wide_many": lambda: graph(39999, 700000)}
+           "wide_few": lambda: graph(1003, 16000),
+           "wide_many": lambda: graph(39999, 700000),
+           "wide_full": lambda: graph(99999, 900000)}
 
 
-@pytest.mark.parametrize("kind", SYSTEMS)
-def test_residual_and_jacobi_are_the_product(kind):
+def kernel(t):
+    """Which of the kernels the layout takes."""
+    per_sm = t.n_slices / torch.cuda.get_device_properties(0).multi_processor_count
+    return "cells" if per_sm > 18 and t.max_width <= 40 else "few" if per_sm <= 8 else "many"
+
+
+@pytest.mark.parametrize("kind,takes", [
+    ("few_slices", "few"), ("many_slices", "many"), ("cells", "cells"), ("cells_2d", "cells"),
+    ("one_slice", "few"), ("wide_few", "few"), ("wide_many", "many"), ("wide_full", "many")])
+def test_residual_and_jacobi_are_the_product(kind, takes):
     m, b, x = SYSTEMS[kind]()
     t = m.topology()
-    assert (t.n_slices > FEW_SLICES) == ("many" in kind)
-    assert (t.max_width > ROW_SLOTS) == kind.startswith("wide")
+    assert kernel(t) == takes and (t.max_width > ROW_SLOTS) == kind.startswith("wide")
     assert torch.equal(bits(residual(m, b, x)), bits(b - m.Ax(x)))
     want = x
     for k in range(1, 4):
