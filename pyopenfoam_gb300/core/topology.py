@@ -48,8 +48,8 @@ class BlockOrder:
     """Cells of a level schedule dealt to resident blocks: block b takes the
     cells [b * per, (b + 1) * per), in level order at cells[ptr[b]:ptr[b + 1]].
     ``share``: chunks of 32 cells that a level has on its busiest block, in the
-    mean over the levels; ``pays``: whether the block walk is then the faster
-    one (see ``WALK_SHARE_MAX``)."""
+    mean over the levels (not counted for blocks of WALK_CELLS_MIN); ``pays``:
+    whether the block walk is the faster one (see ``WALK_SHARE_MAX``)."""
 
     ptr: torch.Tensor
     cells: torch.Tensor
@@ -69,17 +69,17 @@ WALK_CELLS_MIN = 512
 #: busiest block has done its cells, eight chunks of 32 at a time at best, and
 #: in many numberings a front lies on few blocks: the walk over the whole
 #: schedule deals it to all of them.  Time by blocks over time of the whole
-#: schedule, DIC and Gauss-Seidel: share 1.0 (67x59x53 in mesh order) 0.89 and
-#: 0.97, 2.4 (100^3) 0.92 and 1.00, 3.0 (128^3) 1.13 and 1.62, 8.4 (1000x1000
-#: shuffled in runs of 64) 1.42 and 3.3.  Blocks of WALK_CELLS_MIN cells, two
-#: chunks a warp, are the faster walk in every numbering measured (40^3
-#: renumbered, share 3.7, 0.92 and 0.72).
+#: schedule, DIC and Gauss-Seidel: share 1.0 (67x59x53 in mesh order) 0.88 and
+#: 0.86, 2.4 (100^3) 0.90 and 0.91, 3.0 (128^3) 1.13 and 1.57, 8.4 (1000x1000
+#: shuffled in runs of 64) 1.40 and 3.4.  Blocks of WALK_CELLS_MIN cells, two
+#: chunks a warp, are the faster walk in nearly every numbering measured (40^3
+#: renumbered 0.97 and 0.72, 20^3 renumbered 1.04 and 0.78).
 WALK_SHARE_MAX = 2.5
 #: The same where slices have more than four slots a side: such cells take
 #: their values one by one or repeat their row, so that the shorter trips
 #: inside a block count for more.  Share 1.0 (64^3, 10 % renumbered) 0.74 and
-#: 0.50, 3.0 (100^3, 60 % renumbered) 0.72 and 0.74, 3.9 (67x59x53 shuffled in
-#: runs of 4096) 1.19 and 0.88, 8.5 (67x59x53 renumbered) 1.24 and 1.12, 71
+#: 0.51, 3.0 (100^3, 60 % renumbered) 0.67 and 0.75, 3.9 (67x59x53 shuffled in
+#: runs of 4096) 1.18 and 0.89, 8.5 (67x59x53 renumbered) 1.12 and 1.11, 71
 #: (128^3 renumbered) 2.3 and 2.5.
 WALK_SHARE_MAX_WIDE = 3.8
 
@@ -102,7 +102,7 @@ def block_order(level_cells: torch.Tensor | np.ndarray, device: torch.device,
     block = torch.div(cells, per, rounding_mode="floor").to(torch.int16)
     by_block = torch.sort(block, stable=True).indices
     cells, share = cells[by_block], 0.0
-    if level_ptr is not None:
+    if level_ptr is not None and per > WALK_CELLS_MIN:
         n_levels = level_ptr.shape[0] - 1
         level = torch.repeat_interleave(torch.arange(n_levels, device=device), level_ptr.diff(),
                                         output_size=n)

@@ -200,12 +200,12 @@ __global__ void __launch_bounds__(kBlock)
     dic_flow_kernel(gbf_layout L, const double* __restrict__ coef,
                     const double* __restrict__ diag, const int32_t* __restrict__ cells,
                     const int32_t* __restrict__ block_ptr, int per, double* d, GridBarrier* bar,
-                    long long limit) {
+                    long long max_polls) {
   extern __shared__ double dyn[];
   FlowSlots<LOCAL> slots;
   const FlowRange range = flow_begin<LOCAL>(slots, d, L.n_cells, block_ptr, per, dyn);
   const int lane = threadIdx.x & 31;
-  FlowWait<LOCAL> waits(limit);
+  long long polls = 0;
   for (long long at = range.first; at < range.end; at += range.stride) {
     const long long i = at + lane;
     bool done = i >= range.end;
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kBlock)
           done = true;
         }
       }
-      if (waits.pass_end(done, bar, &quit)) break;
+      if (flow_pass_end<!LOCAL>(done, polls, max_polls, bar, &quit)) break;
       if (quit) return;
     }
   }
@@ -510,9 +510,9 @@ static int dic_walk(const char* what, const gbf_layout* L, const double* coef, c
   GBF_CHECK_CUDA(cudaMemsetAsync(d_out, 0xff, sizeof(double) * (size_t)n, s));
   gbf_layout Lc = *L;
   GridBarrier* bar = static_cast<GridBarrier*>(barrier);
-  long long limit = block_ptr ? walk_clocks(n) : kFlowPolls;
+  long long polls = block_ptr ? walk_polls(n) : kFlowPolls;
   void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&cells, (void*)&block_ptr,
-                  &per, &d_out, &bar, &limit};
+                  &per, &d_out, &bar, &polls};
   if (block_ptr) {
     GBF_CHECK_CUDA(launch_walk((const void*)dic_flow_kernel<true>, n_blocks, per, args, barrier, s));
   } else {

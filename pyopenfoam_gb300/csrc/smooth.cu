@@ -195,12 +195,12 @@ __global__ void __launch_bounds__(kBlock)
                    const double* __restrict__ b, const int32_t* __restrict__ cells,
                    const int32_t* __restrict__ block_ptr, int per, int reverse, double omega,
                    const double* __restrict__ x_old, double* x_new, GridBarrier* bar,
-                   long long limit) {
+                   long long max_polls) {
   extern __shared__ double dyn[];
   FlowSlots<LOCAL> slots;
   const FlowRange range = flow_begin<LOCAL>(slots, x_new, L.n_cells, block_ptr, per, dyn);
   const int lane = threadIdx.x & 31;
-  FlowWait<LOCAL> waits(limit);
+  long long polls = 0;
   for (long long at = range.first; at < range.end; at += range.stride) {
     const long long i = at + lane;
     bool done = i >= range.end;
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kBlock)
           done = true;
         }
       }
-      if (waits.pass_end(done, bar, &quit)) break;
+      if (flow_pass_end<!LOCAL>(done, polls, max_polls, bar, &quit)) break;
       if (quit) return;
     }
   }
@@ -635,11 +635,11 @@ static int gauss_seidel_walk(const char* what, const gbf_layout* L, const double
   GBF_CHECK_CUDA(cudaMemsetAsync(scratch, 0xff, sizeof(double) * (size_t)n, s));
   gbf_layout Lc = *L;
   int rev = reverse != 0;
-  long long limit = block_ptr ? walk_clocks(n) : kFlowPolls;
+  long long polls = block_ptr ? walk_polls(n) : kFlowPolls;
   GridBarrier* bar = static_cast<GridBarrier*>(barrier);
   const double* xo = x;
   void* args[] = {&Lc, (void*)&coef, (void*)&diag, (void*)&b, (void*)&cells, (void*)&block_ptr,
-                  &per, &rev, &omega, (void*)&xo, &scratch, &bar, &limit};
+                  &per, &rev, &omega, (void*)&xo, &scratch, &bar, &polls};
   if (block_ptr) {
     const void* k = relax ? (const void*)gs_flow_kernel<true, true>
                           : (const void*)gs_flow_kernel<false, true>;

@@ -80,9 +80,9 @@ inline cudaError_t launch_wavefront(const void* kernel, int grid, void** args, v
 // until their producer stores them; a step polls only the slots it reads.
 // The empty marker is the all-ones bit pattern (a NaN); a NaN result is
 // stored as the canonical NaN so that it cannot read as empty.  Every wait
-// is bounded (by passes, in a block walk by clocks): a warp whose wait runs
-// out sets the barrier's fault word and returns, and the warps that see the
-// fault word return too; the output kernel then writes NaN everywhere.
+// is bounded: after max_polls passes a warp sets the barrier's fault word
+// and returns, and the warps that see the fault word return too; the
+// output kernel then writes NaN everywhere.
 constexpr long long kFlowEmpty = -1LL;
 constexpr long long kFlowPolls = 1LL << 22;  // passes of a warp, a trip through L2 each: > 3 s
 
@@ -146,14 +146,14 @@ struct FlowSlots {
   }
 };
 
-// Clocks that a warp of a block walk over n cells waits for one chunk.  The
-// last block waits for all others: a chain of n cells, one a level, takes 757 ns
-// a cell in the DIC walk and 1020 in the Gauss-Seidel walk, 2100 clocks; four
-// times that, and two seconds for any system.  Passes are no measure here: one
-// that polls shared memory alone takes some 170 ns, and 2^22 of them ran out on
-// chains of about a million cells.
-constexpr long long kWalkClocks = 1LL << 32, kWalkClocksPerCell = 1LL << 13;
-inline long long walk_clocks(int n) { return kWalkClocks + kWalkClocksPerCell * n; }
+// Passes of a warp in a block walk over n cells.  A pass that polls shared
+// memory alone takes some 165 ns, and the last block waits for all others: a
+// chain of n cells, one a level, takes 728 ns a cell in the DIC walk and 884 in
+// the Gauss-Seidel walk, some five passes.  Six times that, and a second for any
+// system (kFlowPolls ran out on chains of about a million cells).  A bound in
+// clocks, looked at every 64th pass, made the Gauss-Seidel sweep of 67x59x53
+// cells 335 us instead of 305.
+inline long long walk_polls(int n) { return (1LL << 23) + 32LL * n; }
 
 // The items a warp takes: 32 at `first`, `stride` further on, up to `end`.
 struct FlowRange {
@@ -192,7 +192,9 @@ inline cudaError_t launch_walk(const void* kernel, int n_blocks, int per, void**
 }
 
 // End of one pass over a chunk: true when every lane is done; false with
-// *quit set when a wait ran out here or elsewhere.
+// *quit set when a wait ran out here or elsewhere.  SLEEP: whether the pass
+// pauses (a walk that polls shared memory does not).
+template <bool SLEEP = true>
 __device__ __forceinline__ bool flow_pass_end(bool done, long long& polls, long long max_polls,
                                               GridBarrier* bar, bool* quit) {
   if (__all_sync(0xffffffffu, done)) return true;
@@ -209,35 +211,8 @@ __device__ __forceinline__ bool flow_pass_end(bool done, long long& polls, long 
   }
   // the pass is bound by the polls' L2 round trip: 0, 16 or 64 ns of sleep
   // measured the same on GB300 (DILU 128^3 2.61-2.62 ms), 256 ns 2 % slower
-  __nanosleep(64);
+  if (SLEEP) __nanosleep(64);
   return false;
 }
-
-// A warp's waits in a walk: over the whole schedule bounded by `limit` passes
-// in all; by blocks (LOCAL), where a pass that polls shared memory does not
-// sleep, by `limit` clocks for each chunk.
-template <bool LOCAL>
-struct FlowWait {
-  long long limit, passes = 0, since = 0;
-
-  __device__ __forceinline__ explicit FlowWait(long long most) : limit(most) {}
-  __device__ __forceinline__ bool pass_end(bool done, GridBarrier* bar, bool* quit) {
-    if constexpr (!LOCAL) {
-      return flow_pass_end(done, passes, limit, bar, quit);
-    } else {
-      if (__all_sync(0xffffffffu, done)) {
-        passes = 0;
-        return true;
-      }
-      if ((++passes & 63) != 0) return false;
-      const long long now = clock64();
-      if (passes == 64) since = now;
-      const bool out = __any_sync(0xffffffffu, now - since > limit);
-      if (out && (threadIdx.x & 31) == 0) atomicExch(&bar->fault, 1);
-      *quit = __any_sync(0xffffffffu, out || *(volatile int*)&bar->fault != 0);
-      return false;
-    }
-  }
-};
 
 }  // namespace gbf

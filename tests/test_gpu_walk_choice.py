@@ -35,7 +35,7 @@ def test_share_and_choice(dims, kind, pays):
     for order, ptr, cells in ((topo.dic_blocks(), sch.ptr[: sch.n_levels + 1], sch.items),
                               (gs.blocks, gs.ptr, gs.cells)):
         want = share_on_host(ptr.cpu().numpy(), cells.cpu().numpy(), order.per)
-        assert order.share == pytest.approx(want, rel=1e-12)
+        assert order.per == WALK_CELLS_MIN or order.share == pytest.approx(want, rel=1e-12)
         assert order.pays == pays == (order.per == WALK_CELLS_MIN or want <= limit)
 
 
