@@ -307,7 +307,13 @@ int gbf_dilu_build_f64(const gbf_layout* L, const double* lower, const double* u
 int gbf_dic_build_flow_f64(const gbf_layout* L, const double* coef, const double* diag,
                            const int32_t* level_cells, double* d_out, void* barrier,
                            void* stream);
-/* DIC with the cells dealt to blocks, as gbf_gauss_seidel_block_f64.          */
+/* DIC with the cells dealt to blocks, as gbf_gauss_seidel_block_f64.  Whether
+ * a block walk is the faster one: gbf_walk_chunks gives the sum over every
+ * `every`-th level, from every / 2 on (host arrays, the cells of a level
+ * ascending), of the chunks of 32 cells on the level's busiest block; up to
+ * some 2.5 a level it is.                                                    */
+int gbf_walk_chunks(int32_t n_levels, const int32_t* level_ptr_h, const int32_t* level_cells_h,
+                    int32_t per, int32_t every, int64_t* chunks_h);
 int gbf_dic_build_block_f64(const gbf_layout* L, const double* coef, const double* diag,
                             const int32_t* block_cells, const int32_t* block_ptr,
                             int32_t n_blocks, int32_t per, double* d_out, void* barrier,

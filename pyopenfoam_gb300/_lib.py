@@ -155,6 +155,8 @@ EXPORTED: dict[str, tuple] = {
     "gbf_gamg_tail_fits": (ctypes.c_int, [_c_i32, _P(_c_i32)]),
     "gbf_gamg_tail_f64": (ctypes.c_int, [_P(GamgLevel), _c_i32, _c_i32, _c_i32, _c_i32, _c_vp,
                                          _c_vp, _c_vp]),
+    "gbf_walk_chunks": (ctypes.c_int, [_c_i32, _c_vp, _c_vp, _c_i32, _c_i32,
+                                       _P(ctypes.c_int64)]),
     "gbf_gs_schedule": (ctypes.c_int, [_c_i32, _c_i32, _c_vp, _c_vp, _c_i32, _c_vp, _c_vp,
                                        _P(_c_i32), _P(_c_i32)]),
     "gbf_gauss_seidel_f64": (ctypes.c_int, [_L, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_vp, _c_i32,

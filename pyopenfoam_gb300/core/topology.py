@@ -31,6 +31,7 @@ class Schedule:
     items: torch.Tensor
     n_levels: int
     max_level_size: int
+    share: float = 0.0  # of the cells dealt to blocks (see BlockOrder)
 
 
 @dataclass
@@ -84,37 +85,47 @@ WALK_SHARE_MAX = 2.5
 WALK_SHARE_MAX_WIDE = 3.8
 
 
-def block_order(level_cells: torch.Tensor | np.ndarray, device: torch.device,
-                level_ptr: torch.Tensor | None = None,
-                max_width: int = 0) -> BlockOrder | None:
-    """The block order of a schedule's cells (each cell once), or None when a
-    block per SM cannot keep its share of them.  Made on the device: the host's
-    sort was 7 ms of a first solve of 10^6 cells.  ``level_ptr`` (device, where
-    each level begins) gives the order its ``share``, which ``max_width`` (slots
-    of the layout's widest slice) judges."""
-    n = level_cells.shape[0]
+def _walk_cells(n: int, device: torch.device) -> int | None:
+    """Cells of a block of a block walk, a block per SM; None when that is more
+    than a block keeps."""
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     per = max(WALK_CELLS_MIN, -(-n // sms))
-    if n == 0 or per > WALK_CELLS_MAX:
+    return per if 0 < n and per <= WALK_CELLS_MAX else None
+
+
+def walk_share(ptr_h: np.ndarray, cells_h: np.ndarray, device: torch.device) -> float:
+    """``BlockOrder.share`` from a schedule's host arrays (the cells of a level
+    ascending), 0.0 where it decides nothing.  Of evenly spaced levels, 64 at
+    least, with some 65536 cells in all: 0.1 to 0.5 ms of a first solve."""
+    n_levels, n = ptr_h.shape[0] - 1, int(ptr_h[-1])
+    per = _walk_cells(n, device) if device.type == "cuda" else None
+    if per is None or per == WALK_CELLS_MIN:
+        return 0.0
+    every = max(1, min(n // 65536, n_levels // 64))
+    chunks = ctypes.c_int64()
+    check(lib().gbf_walk_chunks(n_levels, ptr_h.ctypes.data, cells_h.ctypes.data, per, every,
+                                ctypes.byref(chunks)), "gbf_walk_chunks")
+    return chunks.value / len(range(every // 2, n_levels, every))
+
+
+def block_order(level_cells: torch.Tensor | np.ndarray, device: torch.device,
+                share: float = 0.0, max_width: int = 0) -> BlockOrder | None:
+    """The block order of a schedule's cells (each cell once), or None when a
+    block per SM cannot keep its share of them.  Made on the device: the host's
+    sort was 7 ms of a first solve of 10^6 cells.  ``share`` (``walk_share``) and
+    ``max_width`` (slots of the layout's widest slice) say whether it pays."""
+    n = level_cells.shape[0]
+    per = _walk_cells(n, device)
+    if per is None:
         return None
     n_blocks = -(-n // per)
     cells = torch.as_tensor(level_cells, device=device)
     block = torch.div(cells, per, rounding_mode="floor").to(torch.int16)
-    by_block = torch.sort(block, stable=True).indices
-    cells, share = cells[by_block], 0.0
-    if level_ptr is not None and per > WALK_CELLS_MIN:
-        n_levels = level_ptr.shape[0] - 1
-        level = torch.repeat_interleave(torch.arange(n_levels, device=device), level_ptr.diff(),
-                                        output_size=n)
-        key, count = torch.unique_consecutive(block[by_block].long() * n_levels + level[by_block],
-                                              return_counts=True)
-        most = torch.zeros(n_levels, dtype=torch.int64, device=device)
-        most.scatter_reduce_(0, key % n_levels, (count + 31) // 32, "amax")
-        share = int(most.sum()) / n_levels
+    cells = cells[torch.sort(block, stable=True).indices]
     ptr = np.minimum(np.arange(n_blocks + 1, dtype=np.int64) * per, n).astype(np.int32)
+    limit = WALK_SHARE_MAX if max_width <= 8 else WALK_SHARE_MAX_WIDE
     # the copy from pageable memory waits for the stream, so the order is
     # complete for whichever stream uses it
-    limit = WALK_SHARE_MAX if max_width <= 8 else WALK_SHARE_MAX_WIDE
     return BlockOrder(torch.from_numpy(ptr).to(device), cells, n_blocks, per, share,
                       per == WALK_CELLS_MIN or share <= limit)
 
@@ -258,16 +269,18 @@ class Topology:
                                        cells.ctypes.data, ctypes.byref(nl), ctypes.byref(mx)),
                 "gbf_dic_schedule",
             )
-            self._dic = Schedule(torch.from_numpy(ptr[: nl.value + 1].copy()).to(self.device),
-                                 torch.from_numpy(cells).to(self.device), nl.value, mx.value)
+            ptr = ptr[: nl.value + 1]
+            self._dic = Schedule(torch.from_numpy(ptr.copy()).to(self.device),
+                                 torch.from_numpy(cells).to(self.device), nl.value, mx.value,
+                                 walk_share(ptr, cells, self.device))
         return self._dic
 
     def dic_blocks(self) -> BlockOrder | None:
         """``dic_schedule()``'s cells dealt to blocks (see ``block_order``)."""
         if not self._dic_blocks_made:
             sch = self.dic_schedule()
-            self._dic_blocks = block_order(sch.items[: self.n_cells], self.device,
-                                           sch.ptr[: sch.n_levels + 1], self.max_width)
+            self._dic_blocks = block_order(sch.items[: self.n_cells], self.device, sch.share,
+                                           self.max_width)
             self._dic_blocks_made = True
         return self._dic_blocks
 

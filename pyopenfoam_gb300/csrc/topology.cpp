@@ -286,6 +286,32 @@ extern "C" int gbf_dic_schedule(int32_t n, int32_t nf, const int32_t* own, const
   return GBF_OK;
 }
 
+// Sum over every `every`-th level, from every / 2 on, of ceil(c / 32), c the cells of the level on
+// the block that has most of them (blocks of `per` consecutive cells).  The
+// cells of a level ascend, so those of a block are one run.
+extern "C" int gbf_walk_chunks(int32_t n_levels, const int32_t* level_ptr,
+                               const int32_t* level_cells, int32_t per, int32_t every,
+                               int64_t* chunks) {
+  if (n_levels < 0 || per < 1 || every < 1 || !chunks || (n_levels > 0 && (!level_ptr || !level_cells))) {
+    gbf::set_error("walk_chunks: bad size or NULL pointer");
+    return GBF_ERR_ARG;
+  }
+  int64_t total = 0;
+  for (int64_t l = every / 2; l < n_levels; l += every) {
+    int32_t most = 0, first = level_ptr[l];
+    int64_t end = 0;  // of the run's block
+    for (int32_t i = level_ptr[l]; i < level_ptr[l + 1]; ++i) {
+      if (level_cells[i] < end) continue;
+      most = std::max(most, i - first);
+      first = i;
+      end = ((int64_t)level_cells[i] / per + 1) * per;
+    }
+    total += (std::max(most, level_ptr[l + 1] - first) + 31) / 32;
+  }
+  *chunks = total;
+  return GBF_OK;
+}
+
 extern "C" int gbf_dilu_schedule(int32_t n, int32_t nf, const int32_t* own, const int32_t* nei,
                                  int32_t* level_ptr, int32_t* level_faces, int32_t* n_levels,
                                  int32_t* max_level_size) {

@@ -22,7 +22,7 @@ import torch
 
 from .. import _lib
 from ..core.ldu_matrix import LduMatrix
-from ..core.topology import block_order
+from ..core.topology import block_order, walk_share
 from .preconditioners import DICPreconditioner
 
 __all__ = ["Smoother", "GaussSeidelSmoother", "JacobiSmoother", "DICGSmoother", "gs_sweep",
@@ -59,7 +59,8 @@ class _GsSchedule:
         self.ptr_h = np.ascontiguousarray(ptr[: nl.value + 1])
         self.ptr = torch.from_numpy(self.ptr_h.copy()).to(topo.device)
         self.cells = torch.from_numpy(cells).to(topo.device)
-        self.blocks = block_order(self.cells[:n], topo.device, self.ptr, topo.max_width)
+        self.blocks = block_order(self.cells[:n], topo.device,
+                                  walk_share(self.ptr_h, cells, topo.device), topo.max_width)
 
 
 def _gs_schedule(matrix: LduMatrix, reverse: bool) -> _GsSchedule:
