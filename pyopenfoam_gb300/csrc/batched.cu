@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(BS)
 // slower, 10.8 against 10.1 us), the two sums of a phase share one tree, and
 // what the last tile needs of the state is loaded at the start.  24 systems of
 // 16^3 to 48^3 cells: update phase 10.3 -> 8.0 us, whole solve (448 iterations)
-// 15.9 -> 14.4 ms.  Programmatic dependent launches gave nothing here (the
+// 16.6 -> 15.0 ms.  Programmatic dependent launches gave nothing here (the
 // phases of one wave leave no room for the next kernel's blocks).
 // The persistent form keeps one cell: it has 40 registers for every phase.
 template <bool COH>

@@ -33,7 +33,6 @@
 #include "amul.cuh"
 #include "barrier.cuh"
 #include "exact.cuh"
-#include "wavefront.cuh"
 
 namespace gbf {
 
@@ -736,8 +735,14 @@ static cudaError_t launch_persistent(int grid, const gbf_layout* L, const double
                                      dim3(grid), dim3(kBlock), args, 0, s);
 }
 
-// Systems up to this many cells run the single-launch form under
-// variant 0 (above it the per-iteration launch cost is negligible).
+// Systems up to this many cells run the single-launch form under variant 0.
+// Since the three kernels overlap their launches they are the faster form from
+// about a million cells on hex layouts and throughout on general ones: an
+// iteration with DIC, single launch and three kernels, hex 198360 cells 25.8 and
+// 27.1 us, 499280 37.9 and 42.3, 1000000 64.0 and 64.6, 1560896 95.0 and 84.2,
+// 2080768 123 and 103; renumbered 99360 30.2 and 27.5, 499280 73.6 and 63.0,
+// 2080768 250 and 213.  The line is where it was because the forms sum over
+// other cells: moving it moves the last bits of every solve in between.
 constexpr int kPersistentMaxCells = 1 << 21;
 
 // Whether pcg_resident_kernel takes the system: a hex 3+3 layout, one cell a

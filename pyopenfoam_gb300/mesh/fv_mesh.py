@@ -6,10 +6,11 @@ The reference computes the geometry in Python loops over faces and cells
 (``mesh/mesh_geometry.py:35-395``: hours at 128^3).  Here the same formulas
 run as libgbfoam kernels, one thread per face or cell
 (``gbf_face_geometry_f64``, ``gbf_cell_geometry_f64``,
-``gbf_face_interp_f64``), and so are the cell -> face lists
-(``gbf_cell_faces_device``; a mesh that it does not take, with no faces or a
-cell of more than 4096, goes through the host pass ``gbf_cell_faces``).  Geometry is lazy and cached like the reference's;
-``compute_geometry()`` computes everything at once.
+``gbf_face_interp_f64``).  The cell -> face lists are made by kernels too
+(``gbf_cell_faces_device``); a mesh that they do not take, with no faces or a
+cell of more than 4096, goes through the host pass ``gbf_cell_faces``.
+Geometry is lazy and cached like the reference's; ``compute_geometry()``
+computes everything at once.
 
 Conventions are the reference's: faces are lists of point indices (or a
 CSR pair ``face_ptr`` / ``face_pts``), ``owner`` covers all faces,
